@@ -97,10 +97,13 @@ extern "C" {
  *                    kernels (4, 8 and the FP32 default) never hand a stage to the row
  *                    warps, so the row warps' wait runs out: a test of the timeout path
  *                    that faults nothing.                                      default 0
- *   kernel          -1: the format's default (10 for slices of 32 rows -- SELL-C-sigma
- *                       with C = 32, sell / sell_sorted with vec_len 32 -- without a
- *                       block_nnz, 8 for other SELL-C-sigma, 2 for DIV-RF with 32
- *                       lanes, 4 for the others);
+ *   kernel          -1: the format's default.  With every knob at 0: row tiles (rows sorted by
+ *                       length in windows of 1,024, slices of 32 in tiles of 8 columns, one
+ *                       lane a row) for SELL-C-sigma, and from 3.5 M entries on for the others
+ *                       (FP64; not csr_vec with 1, 2 or 16 lanes, slices of 1 or 2 rows, nor a
+ *                       matrix the layout would pad by more than a third).
+ *                       Otherwise 10 for slices of 32 rows without a block_nnz, 8 for other
+ *                       SELL-C-sigma, 2 for DIV-RF with 32 lanes, 4 for the others;
  *                    0: CTA staged kernel (bulk copy + shared-memory gather, every format);
  *                    1: direct column-major kernel for slices of >= 32 rows;
  *                    2: warp-autonomous staged kernel (CSR, slices of <= 32 rows);

@@ -35,10 +35,10 @@ CUDA_INCLUDE = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(NVC
 GCC_FLAGS = ["-O3", "-march=x86-64-v3", "-fPIC", "-fopenmp", "-std=gnu11", "-Wall", "-Wno-unused-result",
              "-I" + CUDA_INCLUDE]
 
-CU_SOURCES = ["primitives.cu", "convert.cu", "spmv_kernels.cu", "warp_kernels.cu", "div.cu", "fp32.cu", "batch.cu", "select.cu",
+CU_SOURCES = ["primitives.cu", "convert.cu", "spmv_kernels.cu", "warp_kernels.cu", "tile_kernels.cu", "div.cu", "fp32.cu", "batch.cu", "select.cu",
               "mtx.cu", "pack.cu", "sym.cu", "gen.cu", "api.cu"]
 C_SOURCES = ["artgen.c", "mtx_parse.c", "hostcopy.c"]
-HEADERS = ["common.cuh", "primitives.cuh", "internal.h", "mtx_parse.h", "hostcopy.h"]
+HEADERS = ["common.cuh", "primitives.cuh", "internal.h", "tile.h", "mtx_parse.h", "hostcopy.h"]
 
 
 def _newer(src_list, target):

@@ -279,7 +279,7 @@ static int convert_all(Handle & h)
 			break;
 		}
 		SPMV_TRY(convert_csr(h));
-		h.kernels_per_run = (h.num_blocks > 0 || h.num_chunks > 0) ? 1 : 0;
+		h.kernels_per_run = (h.num_blocks > 0 || h.num_chunks > 0 || h.tiles.grid > 0) ? 1 : 0;
 		break;
 	case SPMV_FMT_SELL:
 	case SPMV_FMT_SELL_SORTED:

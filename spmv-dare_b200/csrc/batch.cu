@@ -184,7 +184,8 @@ int build_merged(spmv_batch * b, int32_t count, const int32_t * const * row_ptrs
 	b->total_x = N;
 	b->total_y = M;
 	b->total_nnz = NNZ;
-	b->nblocks = spmv::handle_of(b->merged)->num_blocks;
+	const Handle & mh = *spmv::handle_of(b->merged);
+	b->nblocks = mh.tiles.built ? mh.tiles.grid : mh.num_blocks;
 	return SPMV_OK;
 }
 

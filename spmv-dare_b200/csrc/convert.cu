@@ -454,6 +454,54 @@ static int build_tiled_cols(Handle & h, const int32_t * d_P, int64_t U, int V)
 	return SPMV_OK;
 }
 
+// Row tiles run what the descriptor leaves to the library: any knob, a named kernel, a debug
+// flag, packed columns or tolerance mode selects the kernels those describe.  Slices of 1 or 2
+// rows and csr_vec with 1, 2 or 16 lanes keep kernel 4 (not measured; nothing uses them), and so
+// do matrices of fewer than TILE_ENTRIES entries, which kernel 4 spreads over more warps:
+// csr_naive with 60,895 uneven rows of 19 takes it 6.9 us and row tiles 8.6, 20,036 SELL rows of
+// 57 8.0 and 9.6; from 7.6 M entries on row tiles are the faster (csr_naive 25.9 and 25.1 us
+// there, 50.4 and 37.0 with 10.7 M; sell_sorted 23.9 and 19.3 with 4.1 M).  SELL-C-sigma gains at
+// every size: its other kernels give a slice to a warp or two (1,671 rows 18.9 and 3.6 us).
+constexpr int64_t TILE_ENTRIES = 3500000;
+
+static bool tiles_default(const Handle & h, int V)
+{
+	const spmv_format_desc & d = h.desc;
+	if (d.kernel >= 0 || d.block_nnz || d.block_rows || d.stages || d.ctas_per_sm || d.threads || d.debug_flags ||
+			d.pack_cols || d.row_assign || !d.exact)
+		return false;
+	if (d.format == SPMV_FMT_SELL_C_S)
+		return true;
+	if (h.nnz < TILE_ENTRIES)
+		return false;
+	if (V > 1)
+		return V >= 4;
+	return d.format == SPMV_FMT_CSR_NAIVE || (d.format == SPMV_FMT_CSR_VEC && (d.vec_len == 4 || d.vec_len == 8));
+}
+
+int build_row_tiles(Handle & h, const int32_t * d_P, int V)
+{
+	TileSource t{};
+	t.P = d_P;
+	t.V = V;
+	t.m = h.m;
+	t.entries = V == 1 ? h.nnz : h.stored_elems;
+	t.cols = h.d_ci;
+	t.vals = h.d_v;
+	t.vals_f = h.d_vf;
+	if (h.desc.format == SPMV_FMT_SELL_C_S) {
+		t.cols = h.d_scols;
+		t.vals = h.d_svals;
+		t.ymap = h.d_order;
+	} else if (V > 1) {
+		t.cols = h.d_ja;
+		t.vals = h.d_a;
+		t.ymap = h.desc.format == SPMV_FMT_SELL_SORTED ? h.d_rev : nullptr;
+	}
+	return build_tiles(h.tiles, {t}, h.desc.values == SPMV_VALUES_F32, false, h.num_sms, h.stream,
+			[&h](void ** p, size_t bytes) { return h.alloc((uint8_t **) p, (int64_t) bytes); });
+}
+
 // Kernel choice: -1 = the format's default (the register-tiled warp kernel for slices of 32
 // rows, the tiled warp-specialised kernel for wider SELL-C-sigma slices, the warp-specialised
 // kernel otherwise: the fastest of each on the 4M-row configuration); 0 = CTA
@@ -469,6 +517,13 @@ static int build_tiled_cols(Handle & h, const int32_t * d_P, int64_t U, int V)
 int build_exec(Handle & h, const int32_t * d_P, int64_t U, int V)
 {
 	int k = h.desc.kernel;
+	if (tiles_default(h, V)) {
+		SPMV_TRY(build_row_tiles(h, d_P, V));
+		if (h.tiles.built) {
+			h.exec_kernel = 11;
+			return SPMV_OK;
+		}
+	}
 	if (k < 0) {
 		// measured on the 4M-row matrix: kernel 4 is the fastest for csr_naive (0.193 ms),
 		// csr_vec, and sell / sell_sorted with slices of up to 16 rows; kernel 10 for slices of

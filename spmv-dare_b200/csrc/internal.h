@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "tile.h"
 
 namespace spmv {
 
@@ -102,13 +103,15 @@ struct Handle {
 	int exec_kernel = 0;         // 0 CTA staged, 1 direct sliced, 2 warp-autonomous, 3 pipelined,
 	                             // 4 warp-specialised (gather warps + row warps), 5 CTA staged
 	                             // own-gather, 6 warp-autonomous own-gather, 7 FP32 segmented,
-	                             // 8 warp-specialised over tiled slice columns
+	                             // 8 warp-specialised over tiled slice columns, 9 / 10 tiled warp
+	                             // kernels, 11 row tiles
 	int row_threads = 0;         // kernels 4 and 8: threads of the row warps (the rest gather)
 	int32_t * d_tcols = nullptr; // kernels 8-10: slice column indices, row-major in 8-column tiles
 	int2 * d_items = nullptr;    // kernel 10: work items (slice ranges), heaviest first
 	int64_t num_items = 0;
 	int64_t tile_heavy_min = 0;  // kernel 10: slices at least this long are items of their own
 	unsigned int * d_queue = nullptr;  // kernel 10: work-queue head and finished-warp count
+	TilePlan tiles;              // kernel 11: row tiles
 	uint16_t * d_rassign = nullptr;  // FP32 kernel 4, row_assign 1: local row of each row thread
 	int4 * d_pinfo = nullptr;    // packed columns: per block {16-byte offset, base, bits, bytes}
 	uint32_t * d_pcols = nullptr;  // packed columns: the block streams
@@ -222,6 +225,7 @@ int convert_vector_f2d(const float * in, double * out, int64_t n, cudaStream_t s
 int build_exec(Handle & h, const int32_t * d_P, int64_t U, int V);
 int build_warp_chunks(Handle & h, const int32_t * d_P, int64_t U, int V);
 int build_tile_reg(Handle & h, const int32_t * d_P, int64_t U, int V);
+int build_row_tiles(Handle & h, const int32_t * d_P, int V);
 int launch_warp(Handle & h, const double * d_x, double * d_y, cudaStream_t s);
 
 // ---- SpMV launches

@@ -1,0 +1,58 @@
+// Row tiles (tile_kernels.cu): the execution layout shared by single matrices and batches.
+#pragma once
+
+#include <stdint.h>
+
+#include <functional>
+#include <vector>
+
+#include <cuda_runtime.h>
+
+namespace spmv {
+
+// A converted matrix the layout is built from: CSR rows (V = 1, P = row_ptr) or column-major
+// slices of V rows (V a multiple of 4, P = slice pointer).
+struct TileSource {
+	const int32_t * P;
+	int V;
+	const int32_t * cols;
+	const double * vals;
+	const float * vals_f;        // FP32 variant: the rounded values (long rows read them)
+	const int32_t * ymap;        // row map of sorted slices, or null
+	int64_t m;                   // rows
+	int64_t entries;             // stored entries
+	int64_t x_off, y_off;        // batches: offsets into the concatenated x and y
+};
+
+// A row summed by a whole warp from the format's own arrays.
+struct LongUnit {
+	const int32_t * cols;        // first entry; the others follow `stride` apart
+	const void * vals;
+	int32_t n;
+	int32_t stride;
+	int32_t x_off;
+	int32_t split;               // csr_naive arithmetic (batches)
+	int32_t row;                 // y index
+};
+
+struct TilePlan {
+	bool built = false;
+	bool f32 = false, mixed = false, wide = false, staged = false;
+	int32_t * sptr = nullptr;
+	int32_t * tcols = nullptr;
+	void * vals = nullptr;
+	int32_t * slot_row = nullptr;
+	int32_t * slot_cnt = nullptr;
+	uint8_t * split = nullptr;
+	int4 * ranges = nullptr;
+	LongUnit * longs = nullptr;
+	int64_t nranges = 0, nlong = 0, grid = 0;
+};
+
+// Builds the layout; p.built stays false where it does not pay (padding above a third of the
+// entries) or does not fit 32-bit indices.
+int build_tiles(TilePlan & p, const std::vector<TileSource> & src, bool f32, bool mixed, int num_sms, cudaStream_t s,
+		const std::function<int(void **, size_t)> & alloc);
+int launch_tiles(const TilePlan & p, int format, int lanes, const void * x, void * y, cudaStream_t s);
+
+}  // namespace spmv
