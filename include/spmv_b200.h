@@ -100,7 +100,7 @@ extern "C" {
  *   kernel          -1: the format's default.  With every knob at 0: row tiles (rows sorted by
  *                       length in windows of 1,024, slices of 32 in tiles of 8 columns, one
  *                       lane a row) for SELL-C-sigma, and from 3.5 M entries on for the others
- *                       (FP64; not csr_vec with 1, 2 or 16 lanes, slices of 1 or 2 rows, nor a
+ *                       (FP64 and FP32 CSR; not csr_vec with 1, 2 or 16 lanes, slices of 1 or 2 rows, nor a
  *                       matrix the layout would pad by more than a third).
  *                       Otherwise 10 for slices of 32 rows without a block_nnz, 8 for other
  *                       SELL-C-sigma, 2 for DIV-RF with 32 lanes, 4 for the others;

@@ -460,11 +460,13 @@ static int build_tiled_cols(Handle & h, const int32_t * d_P, int64_t U, int V)
 // do matrices of fewer than TILE_ENTRIES entries, which kernel 4 spreads over more warps:
 // csr_naive with 60,895 uneven rows of 19 takes it 6.9 us and row tiles 8.6, 20,036 SELL rows of
 // 57 8.0 and 9.6; from 7.6 M entries on row tiles are the faster (csr_naive 25.9 and 25.1 us
-// there, 50.4 and 37.0 with 10.7 M; sell_sorted 23.9 and 19.3 with 4.1 M).  SELL-C-sigma gains at
-// every size: its other kernels give a slice to a warp or two (1,671 rows 18.9 and 3.6 us).
+// there, 50.4 and 37.0 with 10.7 M; sell_sorted 23.9 and 19.3 with 4.1 M).  The FP32
+// variant: 14.7 and 18.9 us with 2.6 M entries, 24.0 and 23.2 with 4.7 M, 108 and 68 with 24 M
+// scattered ones, 170 both on the 4M-row matrix.  SELL-C-sigma gains at every size: its other
+// kernels give a slice to a warp or two (1,671 rows 18.9 and 3.6 us).
 constexpr int64_t TILE_ENTRIES = 3500000;
 
-static bool tiles_default(const Handle & h, int V)
+bool tiles_default(const Handle & h, int V)
 {
 	const spmv_format_desc & d = h.desc;
 	if (d.kernel >= 0 || d.block_nnz || d.block_rows || d.stages || d.ctas_per_sm || d.threads || d.debug_flags ||

@@ -1143,6 +1143,14 @@ int convert_f32(Handle & h)
 		h.grid = (int) (g < need ? g : (need > 0 ? need : 1));
 		return SPMV_OK;
 	}
+	if (tiles_default(h, 1)) {
+		SPMV_TRY(build_row_tiles(h, h.d_rp, 1));
+		if (h.tiles.built) {
+			h.exec_kernel = 11;
+			h.kernels_per_run = h.tiles.grid > 0 ? 1 : 0;
+			return SPMV_OK;
+		}
+	}
 	if (h.desc.kernel < 0 || h.desc.kernel == 4) {
 		spmv_format_desc saved = h.desc;
 		h.desc.kernel = 4;
@@ -1305,6 +1313,8 @@ int launch_spmv_f32(Handle & h, const float * d_x, float * d_y, cudaStream_t s)
 {
 	if (h.desc.format == SPMV_FMT_SELL_C_S)
 		return launch_sliced_f32(h, d_x, d_y, s);
+	if (h.exec_kernel == 11)
+		return launch_tiles(h.tiles, h.desc.format, 1, d_x, d_y, s);
 	if (h.exec_kernel == 7) {
 		if (h.num_empty_rows > 0) {
 			zero_rows_f32_kernel<<<(unsigned) ceil_div(h.num_empty_rows, 256), 256, 0, s>>>(h.d_empty_rows,

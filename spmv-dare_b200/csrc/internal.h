@@ -225,6 +225,7 @@ int convert_vector_f2d(const float * in, double * out, int64_t n, cudaStream_t s
 int build_exec(Handle & h, const int32_t * d_P, int64_t U, int V);
 int build_warp_chunks(Handle & h, const int32_t * d_P, int64_t U, int V);
 int build_tile_reg(Handle & h, const int32_t * d_P, int64_t U, int V);
+bool tiles_default(const Handle & h, int V);  // the descriptor leaves the kernel to the library
 int build_row_tiles(Handle & h, const int32_t * d_P, int V);
 int launch_warp(Handle & h, const double * d_x, double * d_y, cudaStream_t s);
 

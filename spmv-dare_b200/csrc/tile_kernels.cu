@@ -194,6 +194,18 @@ __device__ __forceinline__ void load_values(const double * tv, int tw, int lane,
 
 __device__ __forceinline__ void load_values(const float * tv, int tw, int lane, float (&v)[8])
 {
+	if (tw == 8) {
+		const float4 * p = reinterpret_cast<const float4 *>(tv) + lane;
+		#pragma unroll
+		for (int i = 0; i < 2; i++) {
+			const float4 d = __ldcs(p + i * 32);
+			v[4 * i] = d.x;
+			v[4 * i + 1] = d.y;
+			v[4 * i + 2] = d.z;
+			v[4 * i + 3] = d.w;
+		}
+		return;
+	}
 	#pragma unroll
 	for (int p = 0; p < 8; p += 4) {
 		if (p + 3 < tw) {

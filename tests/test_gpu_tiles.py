@@ -113,3 +113,19 @@ def test_infinities_and_nan_as_the_general_kernel(sb, fmt, kw):
     assert np.array_equal(np.isnan(y), np.isnan(ref))
     ok = ~np.isnan(ref)
     assert ok.any() and _bits_equal(y[ok], ref[ok])
+
+
+@pytest.mark.parametrize("rest", [0, 1, 33])
+def test_fp32_rows(sb, orc, rest):
+    """The FP32 variant on row tiles: the sequential Dot2 rows bit for bit."""
+    m = 190 * 1024 + rest
+    r = np.random.default_rng(100 + rest)
+    lengths = r.integers(0, 39, m)
+    for i, k in enumerate([0, 255, 256, 257, 600, 8, 9, 64]):
+        lengths[(3701 * i + 5) % m] = k
+    rp, ci, v, x = _matrix(lengths, rest)
+    assert rp[-1] >= THRESHOLD
+    x32 = x.astype(np.float32)
+    mf = sb.csr_to_format(rp, ci, v, m, N, int(rp[-1]), format="csr_naive", value_type="f32")
+    y = mf.spmv(x32, np.full(m, 1.0, np.float32))
+    assert np.array_equal(y.view(np.uint32), orc.csr_f32_dot2(rp, ci, v.astype(np.float32), x32).view(np.uint32))
