@@ -296,7 +296,8 @@ static int convert_all(Handle & h)
 	}
 	SPMV_CUDA_TRY(cudaStreamSynchronize(h.stream));
 	set_footprints(h);
-	SPMV_TRY(set_x_span(h));
+	if (!h.convert_only)
+		SPMV_TRY(set_x_span(h));
 	h.name = kNames[h.desc.format];
 	if (h.desc.values == SPMV_VALUES_F32)
 		h.name = h.desc.format == SPMV_FMT_SELL_C_S ? "SELL_C_s_F32_Dot2_B200" : "Naive_CSR_F32_Dot2_B200";
@@ -387,6 +388,37 @@ Handle * handle_of(spmv_handle * H)
 {
 	return &H->h;
 }
+
+// spmv_create; convert_only: the format's arrays without an execution schedule (batches build
+// one over all their matrices).
+spmv_handle * create_from_host(const int32_t * row_ptr, const int32_t * col_ind, const double * values, int64_t m,
+		int64_t n, int64_t nnz, int64_t symmetric, int64_t symmetry_expanded, const spmv_format_desc * desc,
+		bool convert_only, int * status)
+{
+	clear_error();
+	int st = SPMV_OK;
+	spmv_handle * H = nullptr;
+	if (!desc) {
+		set_error(SPMV_ERR_ARG, "null format descriptor");
+		st = SPMV_ERR_ARG;
+	} else if (symmetric && !symmetry_expanded) {
+		set_error(SPMV_ERR_UNSUPPORTED, "symmetric matrices have to be expanded to be supported by this format");
+		st = SPMV_ERR_UNSUPPORTED;
+	} else if ((st = check_desc(*desc)) == SPMV_OK) {
+		H = new spmv_handle();
+		H->h.desc = *desc;
+		H->h.convert_only = convert_only;
+		st = create_common(H->h, row_ptr, col_ind, values, m, n, nnz, true, nullptr);
+		if (st != SPMV_OK) {
+			release_handle(H->h);
+			delete H;
+			H = nullptr;
+		}
+	}
+	if (status)
+		*status = st;
+	return H;
+}
 }  // namespace spmv
 
 extern "C" {
@@ -411,28 +443,7 @@ void spmv_format_desc_init(spmv_format_desc * d, int32_t format)
 spmv_handle * spmv_create(const int32_t * row_ptr, const int32_t * col_ind, const double * values, int64_t m, int64_t n,
 		int64_t nnz, int64_t symmetric, int64_t symmetry_expanded, const spmv_format_desc * desc, int * status)
 {
-	spmv::clear_error();
-	int st = SPMV_OK;
-	spmv_handle * H = nullptr;
-	if (!desc) {
-		spmv::set_error(SPMV_ERR_ARG, "null format descriptor");
-		st = SPMV_ERR_ARG;
-	} else if (symmetric && !symmetry_expanded) {
-		spmv::set_error(SPMV_ERR_UNSUPPORTED, "symmetric matrices have to be expanded to be supported by this format");
-		st = SPMV_ERR_UNSUPPORTED;
-	} else if ((st = spmv::check_desc(*desc)) == SPMV_OK) {
-		H = new spmv_handle();
-		H->h.desc = *desc;
-		st = spmv::create_common(H->h, row_ptr, col_ind, values, m, n, nnz, true, nullptr);
-		if (st != SPMV_OK) {
-			spmv::release_handle(H->h);
-			delete H;
-			H = nullptr;
-		}
-	}
-	if (status)
-		*status = st;
-	return H;
+	return spmv::create_from_host(row_ptr, col_ind, values, m, n, nnz, symmetric, symmetry_expanded, desc, false, status);
 }
 
 spmv_handle * spmv_create_device(const int32_t * d_row_ptr, const int32_t * d_col_ind, const double * d_values,

@@ -1,19 +1,23 @@
-// Batched SpMV: hundreds of uneven matrices in one persistent launch (and one CUDA graph).
+// Batched SpMV: hundreds of uneven matrices in one launch (and one CUDA graph).
 //
 // spmv_batch_create converts every matrix with its own format descriptor (the autotuner's
-// pick per matrix: csr_naive, sell, sell_sorted or sell_c_s with their slice parameters),
-// then merges their staged-block tables into one work queue (long units first, so the
-// dependent chains of huge rows start early) with a matrix id per block.  One launch of
-// batch_kernel (spmv_kernels.cu) drains the queue: CTAs claim blocks through an atomic
-// counter, so the load balances across matrices of any size.  x and y of all matrices are
-// concatenated (offsets in spmv_batch_info).
+// pick per matrix: csr_naive, sell, sell_sorted or sell_c_s with their slice parameters).  x and
+// y of all matrices are concatenated (offsets in spmv_batch_info).  Three ways to run:
 //
-// A batch whose matrices are all csr_naive is one SpMV of their block-diagonal matrix over
-// the concatenated x and y: the batch then builds that merged CSR on the device (row
-// pointers and columns shifted by the matrix offsets, each matrix's columns checked against
-// its own n) and runs it as one csr_naive handle -- one launch of the warp-specialised
-// kernel, whose blocks never straddle two matrices' rows.  Every row is still summed in the
-// csr_naive order, so y is bit-identical to the matrices' own handles.
+//   row tiles       the default of mixed batches: one layout (tile_kernels.cu) over the rows of
+//                   all matrices, each slice with its format's arithmetic, ranges of equal cost
+//                   dealt over the whole batch.  48 matrices of 1,000 to 100,000 rows (34 M
+//                   entries, the four formats in turn): 114 us against 486 for the work queue,
+//                   whose CTAs wait at two barriers a block and give a long row to one thread;
+//   work queue      a given block size, stage count or CTA size, tolerance mode, slices of 1 or
+//                   2 rows, or where the layout does not pay: the matrices' staged-block tables
+//                   merged (long units first) with a matrix id per block, drained by one launch
+//                   of batch_kernel (spmv_kernels.cu) through an atomic counter;
+//   block diagonal  all matrices csr_naive: the merged CSR of their block-diagonal matrix (row
+//                   pointers and columns shifted by the matrix offsets, each matrix's columns
+//                   checked against its own n) run as one csr_naive handle.
+//
+// Every row is summed in its format's order: y is bit-identical to the matrices' own handles.
 #include <string.h>
 
 #include <algorithm>
@@ -26,6 +30,9 @@ struct spmv_handle;   // C ABI handle (api.cu)
 
 namespace spmv {
 Handle * handle_of(spmv_handle * H);
+spmv_handle * create_from_host(const int32_t * row_ptr, const int32_t * col_ind, const double * values, int64_t m,
+		int64_t n, int64_t nnz, int64_t symmetric, int64_t symmetry_expanded, const spmv_format_desc * desc,
+		bool convert_only, int * status);
 }
 
 using spmv::Handle;
@@ -45,6 +52,7 @@ struct spmv_batch {
 	int cap = 0, stages = 0, threads = 0, grid = 0;
 	size_t smem = 0;
 	int exact = 1;
+	spmv::TilePlan tiles;              // row tiles over all matrices
 	spmv_handle * merged = nullptr;    // all-csr_naive batches: the block-diagonal matrix
 	// cached CUDA graph of (counter reset + kernel) for one (x, y) pair
 	cudaGraphExec_t graph = nullptr;
@@ -189,10 +197,81 @@ int build_merged(spmv_batch * b, int32_t count, const int32_t * const * row_ptrs
 	return SPMV_OK;
 }
 
+// Row tiles over all matrices of the batch (their format's arrays converted one by one), when
+// the descriptors leave the execution to the library.  b->tiles.built stays false otherwise,
+// and where the layout does not pay or does not fit 32-bit indices.
+int build_batch_tiles(spmv_batch * b, int32_t count, const int32_t * const * row_ptrs, const int32_t * const * col_inds,
+		const double * const * values, const int64_t * ms, const int64_t * ns, const spmv_format_desc * descs)
+{
+	if (count == 0 || descs[0].block_nnz > 0 || descs[0].stages > 0 || descs[0].threads > 0 || !descs[0].exact)
+		return SPMV_OK;
+	int64_t X = 0, Y = 0;
+	for (int32_t i = 0; i < count; i++) {
+		const spmv_format_desc & d = descs[i];
+		const bool sell = d.format == SPMV_FMT_SELL || d.format == SPMV_FMT_SELL_SORTED;
+		if (!(d.format == SPMV_FMT_CSR_NAIVE || d.format == SPMV_FMT_SELL_C_S || (sell && d.vec_len >= 4)) || d.pack_cols ||
+				d.row_assign || d.debug_flags || ms[i] < 0 || ns[i] < 0)
+			return SPMV_OK;
+		X += ns[i];
+		Y += ms[i];
+	}
+	if (X >= INT32_MAX || Y >= INT32_MAX)
+		return SPMV_OK;
+	std::vector<spmv::TileSource> src;
+	int st = SPMV_OK;
+	for (int32_t i = 0; i < count && st == SPMV_OK; i++) {
+		spmv_format_desc d = descs[i];
+		d.kernel = 0;
+		d.block_nnz = b->cap;
+		d.stages = b->stages;
+		d.threads = b->threads;
+		d.exact = 1;
+		d.values = SPMV_VALUES_F64;
+		spmv_handle * H = spmv::create_from_host(row_ptrs[i], col_inds[i], values[i], ms[i], ns[i], row_ptrs[i][ms[i]], 0, 1,
+				&d, true, &st);
+		if (!H)
+			break;
+		b->mats.push_back(H);
+		const Handle & h = *spmv::handle_of(H);
+		spmv::TileSource t = spmv::tile_source(h);
+		t.x_off = b->total_x;
+		t.y_off = b->total_y;
+		src.push_back(t);
+		b->x_off.push_back(b->total_x);
+		b->y_off.push_back(b->total_y);
+		b->total_x += h.n;
+		b->total_y += h.m;
+		b->total_nnz += h.nnz;
+	}
+	if (st == SPMV_OK) {
+		int sms = 0;
+		cudaGetDevice(&b->device);
+		cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
+		st = spmv::build_tiles(b->tiles, src, false, true, sms, b->stream, [b](void ** p, size_t bytes) {
+			return balloc(b, (uint8_t **) p, (int64_t) bytes);
+		});
+	}
+	if (st == SPMV_OK && b->tiles.built) {
+		SPMV_CUDA_TRY(cudaStreamSynchronize(b->stream));
+		b->nblocks = b->tiles.nranges + b->tiles.nlong;
+	}
+	if (st != SPMV_OK || !b->tiles.built) {
+		for (spmv_handle * H : b->mats)
+			spmv_destroy(H);
+		b->mats.clear();
+		b->x_off.clear();
+		b->y_off.clear();
+		b->total_x = b->total_y = b->total_nnz = 0;
+	}
+	return st;
+}
+
 int enqueue(spmv_batch * b, const double * d_x, double * d_y, cudaStream_t s)
 {
 	if (b->merged)
 		return spmv_run_device(b->merged, d_x, d_y, s);
+	if (b->tiles.built)
+		return spmv::launch_tiles(b->tiles, SPMV_FMT_SELL, 1, d_x, d_y, s);
 	SPMV_CUDA_TRY(cudaMemsetAsync(b->d_counter, 0, sizeof(unsigned long long), s));
 	if (b->nblocks == 0)
 		return SPMV_OK;
@@ -257,6 +336,25 @@ spmv_batch * spmv_batch_create(int32_t count, const int32_t * const * row_ptrs, 
 	b->stages = (count > 0 && descs[0].stages > 0) ? descs[0].stages : 2;
 	b->threads = (count > 0 && descs[0].threads > 0) ? descs[0].threads : 256;
 	b->exact = count > 0 ? descs[0].exact : 1;
+	if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) {
+		spmv::set_error(SPMV_ERR_CUDA, "batch: stream creation failed");
+		st = SPMV_ERR_CUDA;
+	}
+	if (st == SPMV_OK)
+		st = build_batch_tiles(b, count, row_ptrs, col_inds, values, ms, ns, descs);
+	if (st != SPMV_OK || b->tiles.built) {
+		if (st == SPMV_OK)
+			st = balloc(b, &b->d_err, 1);
+		if (st == SPMV_OK && cudaMemset(b->d_err, 0, sizeof(int)) != cudaSuccess)
+			st = SPMV_ERR_CUDA;
+		if (st != SPMV_OK) {
+			release(b);
+			b = nullptr;
+		}
+		if (status)
+			*status = st;
+		return b;
+	}
 	std::vector<spmv::BatchMat> hm(count);
 	std::vector<spmv::StagedBlock> blocks;
 	std::vector<int32_t> bmat;
@@ -342,10 +440,6 @@ spmv_batch * spmv_batch_create(int32_t count, const int32_t * const * row_ptrs, 
 		}
 		b->nblocks = (int64_t) ob.size();
 		cudaGetDevice(&b->device);
-		if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) {
-			spmv::set_error(SPMV_ERR_CUDA, "batch: stream creation failed");
-			st = SPMV_ERR_CUDA;
-		}
 		if (st == SPMV_OK)
 			st = balloc(b, &b->d_blocks, b->nblocks);
 		if (st == SPMV_OK)

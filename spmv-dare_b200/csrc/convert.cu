@@ -481,13 +481,22 @@ bool tiles_default(const Handle & h, int V)
 	return d.format == SPMV_FMT_CSR_NAIVE || (d.format == SPMV_FMT_CSR_VEC && (d.vec_len == 4 || d.vec_len == 8));
 }
 
-int build_row_tiles(Handle & h, const int32_t * d_P, int V)
+// The rows of a converted matrix: its CSR rows, or the rows of its slices.
+TileSource tile_source(const Handle & h)
 {
 	TileSource t{};
-	t.P = d_P;
-	t.V = V;
+	t.P = h.d_rp;
+	t.V = 1;
+	if (h.desc.format == SPMV_FMT_SELL_C_S) {
+		t.P = h.d_sptr32;
+		t.V = h.desc.sellcs_c;
+	} else if (h.desc.format == SPMV_FMT_SELL || h.desc.format == SPMV_FMT_SELL_SORTED) {
+		t.P = h.d_rcp;
+		t.V = h.desc.vec_len;
+	}
 	t.m = h.m;
-	t.entries = V == 1 ? h.nnz : h.stored_elems;
+	t.split = h.desc.format == SPMV_FMT_CSR_NAIVE;
+	t.entries = t.P == h.d_rp ? h.nnz : h.stored_elems;
 	t.cols = h.d_ci;
 	t.vals = h.d_v;
 	t.vals_f = h.d_vf;
@@ -495,12 +504,17 @@ int build_row_tiles(Handle & h, const int32_t * d_P, int V)
 		t.cols = h.d_scols;
 		t.vals = h.d_svals;
 		t.ymap = h.d_order;
-	} else if (V > 1) {
+	} else if (t.P == h.d_rcp) {
 		t.cols = h.d_ja;
 		t.vals = h.d_a;
 		t.ymap = h.desc.format == SPMV_FMT_SELL_SORTED ? h.d_rev : nullptr;
 	}
-	return build_tiles(h.tiles, {t}, h.desc.values == SPMV_VALUES_F32, false, h.num_sms, h.stream,
+	return t;
+}
+
+int build_row_tiles(Handle & h)
+{
+	return build_tiles(h.tiles, {tile_source(h)}, h.desc.values == SPMV_VALUES_F32, false, h.num_sms, h.stream,
 			[&h](void ** p, size_t bytes) { return h.alloc((uint8_t **) p, (int64_t) bytes); });
 }
 
@@ -518,9 +532,11 @@ int build_row_tiles(Handle & h, const int32_t * d_P, int V)
 // sum them from registers, tiles one ahead, x transposed between lanes (no shared memory).
 int build_exec(Handle & h, const int32_t * d_P, int64_t U, int V)
 {
+	if (h.convert_only)
+		return SPMV_OK;
 	int k = h.desc.kernel;
 	if (tiles_default(h, V)) {
-		SPMV_TRY(build_row_tiles(h, d_P, V));
+		SPMV_TRY(build_row_tiles(h));
 		if (h.tiles.built) {
 			h.exec_kernel = 11;
 			return SPMV_OK;

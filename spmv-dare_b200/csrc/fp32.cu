@@ -1144,7 +1144,7 @@ int convert_f32(Handle & h)
 		return SPMV_OK;
 	}
 	if (tiles_default(h, 1)) {
-		SPMV_TRY(build_row_tiles(h, h.d_rp, 1));
+		SPMV_TRY(build_row_tiles(h));
 		if (h.tiles.built) {
 			h.exec_kernel = 11;
 			h.kernels_per_run = h.tiles.grid > 0 ? 1 : 0;

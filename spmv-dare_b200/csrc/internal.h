@@ -174,6 +174,8 @@ struct Handle {
 	float * d_xf = nullptr;
 	float * d_yf = nullptr;
 
+	bool convert_only = false;          // a batch's matrix: no execution schedule of its own
+
 	std::vector<void *> allocations;    // everything above, freed by destroy
 	double mem_footprint = 0;
 	double csr_mem_footprint = 0;
@@ -226,7 +228,8 @@ int build_exec(Handle & h, const int32_t * d_P, int64_t U, int V);
 int build_warp_chunks(Handle & h, const int32_t * d_P, int64_t U, int V);
 int build_tile_reg(Handle & h, const int32_t * d_P, int64_t U, int V);
 bool tiles_default(const Handle & h, int V);  // the descriptor leaves the kernel to the library
-int build_row_tiles(Handle & h, const int32_t * d_P, int V);
+TileSource tile_source(const Handle & h);
+int build_row_tiles(Handle & h);
 int launch_warp(Handle & h, const double * d_x, double * d_y, cudaStream_t s);
 
 // ---- SpMV launches

@@ -11,7 +11,7 @@
 namespace spmv {
 
 // A converted matrix the layout is built from: CSR rows (V = 1, P = row_ptr) or column-major
-// slices of V rows (V a multiple of 4, P = slice pointer).
+// slices of V rows (P = slice pointer).
 struct TileSource {
 	const int32_t * P;
 	int V;
@@ -21,6 +21,7 @@ struct TileSource {
 	const int32_t * ymap;        // row map of sorted slices, or null
 	int64_t m;                   // rows
 	int64_t entries;             // stored entries
+	bool split;                  // csr_naive arithmetic: product and sum rounded separately
 	int64_t x_off, y_off;        // batches: offsets into the concatenated x and y
 };
 

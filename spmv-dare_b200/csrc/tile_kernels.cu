@@ -86,17 +86,8 @@ template <>
 struct RowSum<Sum::FMA> : FusedSum {};
 
 template <>
-struct RowSum<Sum::MIXED> {                     // batches: the slice's own choice of the two
-	using T = double;
-	double s = 0.0;
+struct RowSum<Sum::MIXED> : FusedSum {          // batches: either of the two, by slice
 	bool split = false;
-	template <int J, bool FULL>
-	__device__ __forceinline__ void step(int k, int n, double v, double x)
-	{
-		const bool in = FULL || k < n;
-		s = split ? __dadd_rn(s, in ? __dmul_rn(v, x) : -0.0) : __fma_rn(in ? v : -0.0, in ? x : 1.0, s);
-	}
-	__device__ __forceinline__ double total(int) const { return s; }
 };
 
 template <int L>
@@ -291,6 +282,25 @@ __device__ __forceinline__ void tile_steps(A & acc, int k0, int n, const T (&v)[
 	acc.template step<5, FULL>(k0 + 5, n, v[5], Y[1]);
 	acc.template step<6, FULL>(k0 + 6, n, v[6], Y[2]);
 	acc.template step<7, FULL>(k0 + 7, n, v[7], Y[3]);
+}
+
+// tile_steps for the warp's tile, without masks where no row of it ends.
+template <Sum S, typename A, typename T>
+__device__ __forceinline__ void add_tile(A & acc, bool full, int k0, int n, const T (&v)[8], uint32_t xrow)
+{
+	if constexpr (S == Sum::MIXED) {
+		if (acc.split) {
+			SplitSum t;
+			t.s = acc.s;
+			add_tile<Sum::NAIVE>(t, full, k0, n, v, xrow);
+			acc.s = t.s;
+			return;
+		}
+	}
+	if (full)
+		tile_steps<true>(acc, k0, n, v, xrow);
+	else
+		tile_steps<false>(acc, k0, n, v, xrow);
 }
 
 // Asynchronous copy of one x entry into shared memory.
@@ -563,10 +573,8 @@ __global__ void __launch_bounds__(TILE_THREADS, MINB) tile_kernel(TileArgs a)
 			asm volatile("cp.async.wait_group 1;" ::: "memory");
 		__syncwarp();
 		const int k0 = (t0 - b) >> 5;
-		if (__all_sync(0xffffffffu, k0 + 8 <= (n & WHOLE)))
-			tile_steps<true>(acc, k0, n, vt, xrow + buf);
-		else
-			tile_steps<false>(acc, k0, n, vt, xrow + buf);
+		const bool full = __all_sync(0xffffffffu, k0 + 8 <= (n & WHOLE));
+		add_tile<S>(acc, full, k0, n, vt, xrow + buf);
 		if (!AHEAD)
 			load_values(vals + t1, q >> TILE_BITS & 15, lane, vn);
 		if constexpr (STAGED)
@@ -717,7 +725,7 @@ __global__ void tile_fill_kernel(TileSource s, int64_t slice0, int64_t nslices, 
 	if (src >= 0)
 		source_row(s, src, start, stride, cnt);
 	if (split && r == 0)
-		split[sl] = s.V == 1;
+		split[sl] = s.split;
 	int32_t pad = cnt > 0 ? s.cols[start] : 0;      // columns of the padding: read, never summed
 	for (int k8 = 0; k8 < W; k8 += 8) {
 		const int tw = W - k8 < 8 ? W - k8 : 8;
@@ -804,7 +812,7 @@ __global__ void long_units_kernel(TileSource s, const T * vals, int long_min, in
 	u.n = cnt;
 	u.stride = stride;
 	u.x_off = (int32_t) s.x_off;
-	u.split = s.V == 1;
+	u.split = s.split;
 	u.row = (int32_t) (s.y_off + (s.ymap ? s.ymap[i] : i));
 	out[atomicAdd(next, 1)] = u;
 }
@@ -888,8 +896,13 @@ int build_tiles(TilePlan & p, const std::vector<TileSource> & src, bool f32, boo
 				break;
 			}
 	}
-	const int long_min = (int) lm;
-	if (lm >= (1 << 21) - 2 || nslots > INT32_MAX - 64)
+	std::vector<int> long_min;                  // a batch's matrices: four times their own mean at least
+	for (const TileSource & t : src) {
+		const int64_t own = src.size() > 1 && t.m > 0 ? 4 * (t.entries / t.m) : 0;
+		lm = lm > (1 << 21) - 3 ? (1 << 21) - 3 : lm;
+		long_min.push_back((int) (own > lm && own < (1 << 21) - 3 ? own : lm));
+	}
+	if (4 * mean >= (1 << 21) - 3 || nslots > INT32_MAX - 64)
 		return SPMV_OK;
 	DevBuf d_src, width, sptr64;
 	SPMV_TRY(d_src.alloc(nslots * sizeof(int32_t), s));
@@ -900,7 +913,7 @@ int build_tiles(TilePlan & p, const std::vector<TileSource> & src, bool f32, boo
 	for (size_t i = 0; i < src.size(); i++) {
 		if (src[i].m == 0)
 			continue;
-		tile_sort_kernel<<<(unsigned) ceil_div(src[i].m, TILE_WINDOW), TILE_WINDOW / 2, 0, s>>>(src[i], long_min, slot0[i],
+		tile_sort_kernel<<<(unsigned) ceil_div(src[i].m, TILE_WINDOW), TILE_WINDOW / 2, 0, s>>>(src[i], long_min[i], slot0[i],
 				ceil_div(src[i].m, 32) * 32, d_src.as<int32_t>(), p.slot_row, p.slot_cnt, width.as<int64_t>(), cnt.as<int>());
 		SPMV_CUDA_TRY(cudaGetLastError());
 	}
@@ -931,12 +944,12 @@ int build_tiles(TilePlan & p, const std::vector<TileSource> & src, bool f32, boo
 			tile_fill_kernel<float><<<g, 256, 0, s>>>(src[i], slot0[i] / 32, n, d_src.as<int32_t>(), p.sptr, p.tcols,
 					(float *) p.vals, p.split);
 			if (nlong > 0)
-				long_units_kernel<float><<<gl, 256, 0, s>>>(src[i], src[i].vals_f, long_min, cnt.as<int>() + 1, p.longs);
+				long_units_kernel<float><<<gl, 256, 0, s>>>(src[i], src[i].vals_f, long_min[i], cnt.as<int>() + 1, p.longs);
 		} else {
 			tile_fill_kernel<double><<<g, 256, 0, s>>>(src[i], slot0[i] / 32, n, d_src.as<int32_t>(), p.sptr, p.tcols,
 					(double *) p.vals, p.split);
 			if (nlong > 0)
-				long_units_kernel<double><<<gl, 256, 0, s>>>(src[i], src[i].vals, long_min, cnt.as<int>() + 1, p.longs);
+				long_units_kernel<double><<<gl, 256, 0, s>>>(src[i], src[i].vals, long_min[i], cnt.as<int>() + 1, p.longs);
 		}
 		SPMV_CUDA_TRY(cudaGetLastError());
 	}

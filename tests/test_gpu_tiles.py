@@ -129,3 +129,28 @@ def test_fp32_rows(sb, orc, rest):
     mf = sb.csr_to_format(rp, ci, v, m, N, int(rp[-1]), format="csr_naive", value_type="f32")
     y = mf.spmv(x32, np.full(m, 1.0, np.float32))
     assert np.array_equal(y.view(np.uint32), orc.csr_f32_dot2(rp, ci, v.astype(np.float32), x32).view(np.uint32))
+
+
+def test_batch_of_edges(sb, orc):
+    """A mixed batch: empty and one-row matrices, sizes around slices and windows, long rows."""
+    import torch
+
+    r = np.random.default_rng(21)
+    mats, fmts = [], []
+    for i, m in enumerate([1, 0, 33, 1024, 1025, 2050, 5000, 31, 64, 3000, 7, 4097]):
+        lengths = r.integers(0, 60, m)
+        if m:
+            lengths[m // 2] = 300 + 211 * i
+        rp, ci, v, x = _matrix(lengths, i)
+        mats.append((rp, ci, v, m, N))
+        fmts.append([("csr_naive", {}), ("sell", dict(vec_len=4)), ("sell_sorted", dict(vec_len=8)),
+                     ("sell_c_s", dict(sellcs_c=32, sellcs_sigma=512))][i % 4])
+    b = sb.Batch(mats, [dict(kw, format=f) for f, kw in fmts])
+    x = r.uniform(-1, 1, b.total_x)
+    yd = torch.full((b.total_y,), 5.0, dtype=torch.float64, device="cuda")
+    b.spmv(torch.from_numpy(x).cuda(), yd)
+    b.sync()
+    y = yd.cpu().numpy()
+    for (rp, ci, v, m, n), (f, kw), xo, yo in zip(mats, fmts, b.x_offsets, b.y_offsets):
+        if m:
+            assert _bits_equal(y[yo:yo + m], _expected(orc, f, kw, rp, ci, v, x[xo:xo + n])), (m, f)
