@@ -103,7 +103,10 @@ extern "C" {
  *                       (FP64 and FP32 CSR; not csr_vec with 1, 2 or 16 lanes, slices of 1 or 2 rows, nor a
  *                       matrix the layout would pad by more than a third).
  *                       Otherwise 10 for slices of 32 rows without a block_nnz, 8 for other
- *                       SELL-C-sigma, 2 for DIV-RF with 32 lanes, 4 for the others;
+ *                       SELL-C-sigma, 4 for the others.  DIV-RF: the segment decoder up to 32
+ *                       lanes (warps decode runs of a packet from places noted at
+ *                       conversion) when block_nnz, stages and ctas_per_sm are 0, else 2 with
+ *                       32 lanes and 0 otherwise;
  *                    0: CTA staged kernel (bulk copy + shared-memory gather, every format);
  *                    1: direct column-major kernel for slices of >= 32 rows;
  *                    2: warp-autonomous staged kernel (CSR, slices of <= 32 rows);

@@ -948,6 +948,355 @@ __global__ void __launch_bounds__(DIVW_WARPS * 32, MINB) div_warp_kernel(DivArgs
 	}
 }
 
+// ------------------------------------------------------------------ segment decoder
+// The default for up to 32 lanes.  One CTA per packet, its warps taking segments of the packet
+// independently of each other.  A segment is a run of whole positions of one group (all L lanes
+// of unique values, about div_segment_entries(L) coordinates), a part of one position's
+// coordinates where rf is large, or the group's last, incomplete position.  The conversion
+// leaves beside the stream where each lane's payload starts in a segment and the value it
+// continues from (div_sync_kernel; 0.2 bytes an entry with 4 lanes, 0.8 with 32), so no warp
+// waits for another and a thread never walks a lane alone.  32 unique values a step: code bytes
+// from 32 neighbouring bytes, the payloads found by a scan of their lengths over the lane's
+// positions in the warp and turned into values by a scan of the differences; then the step's
+// rf * 32 coordinates, 32 neighbouring ones at a time, each taking its value from the thread
+// that decoded it.  Row sums in shared memory, stored as in the other decoders.
+//
+// What bounds it: the L1 pipe (x is read in value order, a line an entry; shared FP64 additions
+// are compare-and-swap loops, about 40 us of 20 M entries) and instruction issue (some 180 a 32
+// entries); DRAM is 9% busy.  Measured in a loop over three matrices, before and now: 4 lanes,
+// 20 M distinct values 244 -> 203 us; 8 M entries of 300 values 454 -> 98 us with 32 lanes (groups
+// of few values left most lanes of the warp decoder idle) and 2,286 -> 91 with 4 (one thread
+// walked a value's coordinates); 32 lanes, distinct values, 4,096-value packets 243 -> 200.
+// Tried: no lookahead 385, lines asked of L1 a segment ahead 303, and the next step's payload
+// and x loads under way 203-211; CTAs of 256 threads 235, of 512 285 (packets of some 5,000
+// entries are their unit of balance); row sums a warp 236; segments of 512 entries 242.
+constexpr int DIVS_THREADS = 128;
+
+__host__ __device__ __forceinline__ int div_segment_entries(int L)
+{
+	return L <= 16 ? 256 : 16 * L;
+}
+
+struct DivSegArgs {
+	const uint8_t * data;
+	const uint8_t * end;         // of the stream
+	const int64_t * pkt_off;
+	const int4 * meta;
+	const int32_t * pkt_seg;     // first segment of each packet
+	const int4 * segs;           // two a segment: {first code, unique values, rf, first coordinate},
+	                             // {first and end of its coordinates, index of its values or -1, incomplete position}
+	const uint32_t * seg_off;    // L a segment: payload byte of each lane
+	const uint64_t * seg_val;    // L a segment that continues a lane: its last value
+	const double * x;
+	double * y;
+};
+
+// Inclusive sum over the threads of a lane (t % L) up to this one.
+template <int L, typename T>
+__device__ __forceinline__ T lane_inclusive_scan(T v, int t)
+{
+	#pragma unroll
+	for (int d = L; d < 32; d <<= 1) {
+		const T o = __shfl_up_sync(0xffffffffu, v, d);
+		if (t >= d)
+			v += o;
+	}
+	return v;
+}
+
+// Geometry of a packet's coordinates: cb bytes each, the row in the low row_bits.
+struct Coords {
+	const uint8_t * base;
+	int cb, row_bits;
+	uint32_t mask, rmask, cmask;
+	__device__ __forceinline__ Coords(const uint8_t * p, int rb, int colb)
+	{
+		base = p;
+		row_bits = rb;
+		cb = (rb + colb + 7) >> 3;
+		mask = cb >= 4 ? ~0u : (1u << (8 * cb)) - 1u;
+		rmask = (1u << rb) - 1u;                         // at most 8 bits
+		cmask = colb >= 32 ? ~0u : (1u << colb) - 1u;
+	}
+	// row and column of coordinate i: up to 4 bytes from two 32-bit words and a funnel shift
+	__device__ __forceinline__ void get(int64_t i, uint32_t & row, uint32_t & col) const
+	{
+		const uint8_t * p = base + i * cb;
+		if (cb > 4) {
+			const uint64_t c = ld_bytes(p, cb);
+			row = (uint32_t) c & rmask;
+			col = (uint32_t) (c >> row_bits) & cmask;
+			return;
+		}
+		const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+		const uint32_t * w = reinterpret_cast<const uint32_t *>(a & ~(uintptr_t) 3);
+		const uint32_t c = __funnelshift_r(__ldg(w), __ldg(w + 1), (uint32_t) (a & 3) * 8u) & mask;
+		row = c & rmask;
+		col = c >> row_bits;
+	}
+};
+
+// A value difference: len <= 8 little-endian payload bytes, shifted.  The words that hold 8
+// bytes at p (up to 11 bytes past it are read), and the difference they code.
+struct Payload {
+	uint32_t w0 = 0, w1 = 0, w2 = 0, sh = 0;
+	__device__ __forceinline__ void load(const uint8_t * p)
+	{
+		const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+		const uint32_t * w = reinterpret_cast<const uint32_t *>(a & ~(uintptr_t) 3);
+		sh = (uint32_t) (a & 3) * 8u;
+		w0 = __ldg(w);
+		w1 = __ldg(w + 1);
+		w2 = __ldg(w + 2);
+	}
+	__device__ __forceinline__ uint64_t diff(int code) const
+	{
+		const int len = code & 15;
+		const uint64_t v = (uint64_t) __funnelshift_r(w1, w2, sh) << 32 | __funnelshift_r(w0, w1, sh);
+		const int drop = 64 - 8 * len;
+		return len ? (v << drop) >> drop << ((code >> 4) << 2) : 0;
+	}
+};
+
+__device__ __forceinline__ uint64_t diff_at(const uint8_t * p, int code)
+{
+	Payload w;
+	w.load(p);
+	return w.diff(code);
+}
+
+__device__ __forceinline__ void prefetch_l1(const uint8_t * p, const uint8_t * end)
+{
+	if (p < end)
+		asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
+}
+
+template <int L>
+__global__ void __launch_bounds__(DIVS_THREADS, 6) div_segment_kernel(DivSegArgs a)
+{
+	__shared__ double ys[DEC_MAX_ROWS];
+	const int64_t p = blockIdx.x;
+	const int t = threadIdx.x & 31, l = t & (L - 1);
+	const uint8_t * h = a.data + a.pkt_off[p];
+	const int64_t nv = ld_u32(h + 0), nu = ld_u32(h + 4), nrows = ld_u32(h + 8);
+	const int64_t row_min = ld_u32(h + 12), col_min = ld_u32(h + 16);
+	const int row_bits = h[20], col_bits = h[21];
+	const int64_t nrf = ld_u32(h + 24);
+	const Coords coords(h + 28 + 4 * L + 8 * nrf, row_bits, col_bits);
+	const uint8_t * codes = coords.base + coords.cb * nv;
+	const uint8_t * lanes = codes + nu;
+	const double * __restrict__ x = a.x + col_min;
+	const int s_end = a.pkt_seg[p + 1];
+	constexpr int WARPS = DIVS_THREADS / 32;
+	int s = a.pkt_seg[p] + (threadIdx.x >> 5);
+	// a segment's descriptor and places, and its lines asked of L1: the warp runs one ahead
+	int4 A, B;
+	uint32_t off = 0;
+	uint64_t val = 0;
+	auto fetch = [&](int sg) {
+		if (sg >= s_end)
+			return;
+		A = __ldg(a.segs + 2 * (int64_t) sg);
+		B = __ldg(a.segs + 2 * (int64_t) sg + 1);
+		off = __ldg(a.seg_off + (int64_t) sg * L + l);
+		val = B.z >= 0 ? __ldg(a.seg_val + (int64_t) B.z * L + l) : 0;
+		// payloads: 8 bytes a position at most, the lane's 32 / L threads a line each
+		const int pay = (A.y + L - 1) / L * 8;
+		for (int o = t / L * 128; o < pay; o += 32 / L * 128)
+			prefetch_l1(lanes + off + o, a.end);
+		const uint8_t * c = codes + A.x;
+		if (t * 128 < A.y + 127)
+			prefetch_l1(c + (t * 128 < A.y ? t * 128 : A.y - 1), a.end);
+		const uint8_t * q = coords.base + ((int64_t) A.w + (A.y > 32 ? 0 : B.x)) * coords.cb;
+		const int bytes = (A.y > 32 ? A.y * A.z : B.y - B.x) * coords.cb;
+		for (int o = t * 128; o < bytes + 127; o += 32 * 128)
+			prefetch_l1(q + (o < bytes ? o : bytes - 1), a.end);
+	};
+	fetch(s);
+	for (int r = threadIdx.x; r < nrows && r < DEC_MAX_ROWS; r += blockDim.x)
+		ys[r] = 0.0;
+	__syncthreads();
+	while (s < s_end) {
+		const int first = A.x, nuniq = A.y, rf = A.z, coord0 = A.w, part0 = B.x, part1 = B.y;
+		const bool rest = B.w != 0;
+		uint32_t at = off;
+		uint64_t last = val;
+		s += WARPS;
+		fetch(s);
+		const int per = rest ? rf : L * rf;
+		const float inv = 1.0f / (float) per;
+		if (rf == 1) {
+			// one coordinate a value: the next step's payload words, row and x are under way while
+			// this step's values are scanned and added
+			int code = t < nuniq ? __ldg(codes + first + t) : 0;
+			int code1 = 32 + t < nuniq ? __ldg(codes + first + 32 + t) : 0;
+			Payload w, w1;
+			uint32_t row = 0, row1 = 0, col;
+			double xv = 0.0, xv1 = 0.0;
+			auto ahead = [&](int u, int cd, Payload & pw, uint32_t & r, double & xx) {
+				const int len = cd & 15, ends = lane_inclusive_scan<L>(len, t);
+				pw.load(lanes + at + (ends - len));
+				at += (uint32_t) __shfl_sync(0xffffffffu, ends, 32 - L + l);
+				if (u + t < nuniq) {
+					coords.get(coord0 + u + t, r, col);
+					xx = __ldg(x + col);
+				}
+			};
+			ahead(0, code, w, row, xv);
+			for (int u0 = 0; u0 < nuniq; u0 += 32) {
+				if (u0 + 32 < nuniq)
+					ahead(u0 + 32, code1, w1, row1, xv1);
+				const int code2 = u0 + 64 + t < nuniq ? __ldg(codes + first + u0 + 64 + t) : 0;
+				const uint64_t v = last + lane_inclusive_scan<L>(w.diff(code), t);
+				last = __shfl_sync(0xffffffffu, v, 32 - L + l);
+				if (u0 + t < nuniq)
+					atomicAdd(&ys[row], __longlong_as_double((long long) v) * xv);
+				code = code1;
+				code1 = code2;
+				w = w1;
+				row = row1;
+				xv = xv1;
+			}
+			continue;
+		}
+		for (int u0 = 0; u0 < nuniq; u0 += 32) {
+			const bool in = u0 + t < nuniq;
+			const int code = in ? __ldg(codes + first + u0 + t) : 0;
+			const int len = code & 15;
+			const int ends = lane_inclusive_scan<L>(len, t);
+			const uint64_t v = last + lane_inclusive_scan<L>(diff_at(lanes + at + (ends - len), code), t);
+			// the last thread of the lane hands its place and value to the next step
+			at += (uint32_t) __shfl_sync(0xffffffffu, ends, 32 - L + l);
+			last = __shfl_sync(0xffffffffu, v, 32 - L + l);
+			const double vd = __longlong_as_double((long long) v);
+			const bool whole = nuniq > 32;
+			const int left = nuniq - u0 < 32 ? nuniq - u0 : 32;
+			const int c0 = whole ? 0 : part0, c1 = whole ? left * rf : part1;
+			for (int cc = c0; cc < c1; cc += 32) {
+				const int e = cc + t;
+				const bool on = e < c1;
+				uint32_t row = 0, col;
+				double xe = 0.0;
+				if (on) {
+					coords.get((int64_t) coord0 + u0 * rf + e, row, col);
+					xe = __ldg(x + col);
+				}
+				// the thread that holds the coordinate's value: e / rf in an incomplete position,
+				// else lane e % L of position e / (L rf)
+				int q = (int) ((float) e * inv);
+				q -= q * per > e;
+				q += (q + 1) * per <= e;
+				const int from = rest ? q : q * L + ((e - q * per) & (L - 1));
+				const double ve = __shfl_sync(0xffffffffu, vd, from & 31);
+				if (on)
+					atomicAdd(&ys[row], ve * xe);
+			}
+		}
+	}
+	__syncthreads();
+	const int4 mt = a.meta[p];
+	for (int64_t r = (int64_t) mt.x + threadIdx.x; r < (int64_t) mt.y; r += blockDim.x) {
+		const int64_t rel = r - row_min;
+		if (rel < 0 || rel >= nrows) {
+			a.y[r] = 0.0;                                // empty rows between packets
+		} else if ((rel == 0 && (mt.z & 1)) || (rel == nrows - 1 && (mt.z & 2))) {
+			atomicAdd(&a.y[r], ys[rel]);                 // a row split across packets
+		} else {
+			a.y[r] = ys[rel];
+		}
+	}
+}
+
+// Segments of a group of u unique values of rf coordinates: whole positions in runs of `np`,
+// or one by one in `parts` of their coordinates; then the incomplete position in parts.
+struct GroupSegments {
+	int64_t dv, md, np, parts, full, rest;
+	__device__ __forceinline__ GroupSegments(int64_t u, int64_t rf, int L)
+	{
+		const int64_t S = div_segment_entries(L), step = 32 / L;
+		dv = u / L;
+		md = u % L;
+		parts = 1;
+		np = 1;
+		if (L * rf > S) {
+			parts = (L * rf + S - 1) / S;
+		} else {
+			np = S / (L * rf);
+			np = np >= step ? np / step * step : np;     // steps of 32 values
+		}
+		full = (dv + np - 1) / np * parts;
+		rest = (md * rf + S - 1) / S;
+	}
+};
+
+__global__ void div_seg_count_kernel(const int64_t * g_u, const int32_t * g_rf, int64_t G, int L, int64_t * count,
+		int64_t * nval)
+{
+	const int64_t g = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
+	if (g >= G)
+		return;
+	const GroupSegments k(g_u[g], g_rf[g], L);
+	count[g] = k.full + k.rest;
+	nval[g] = (k.full > 0 ? k.full - k.parts : 0) + (k.dv > 0 ? k.rest : 0);     // segments that continue a lane
+}
+
+__global__ void div_pkt_seg_kernel(const int32_t * pk_g0, const int64_t * seg_base, int64_t NP, int32_t * pkt_seg)
+{
+	const int64_t p = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
+	if (p <= NP)
+		pkt_seg[p] = (int32_t) seg_base[pk_g0[p]];
+}
+
+// One thread per (segment, lane).
+__global__ void div_sync_kernel(const int64_t * seg_base, const int64_t * val_base, int64_t G, int64_t nseg, int L,
+		const int64_t * g_u, const int32_t * g_rf, const int64_t * g_ustart, const int64_t * g_start,
+		const int32_t * g_pkt, const int32_t * pk_g0, const int32_t * pk_j, const int64_t * gl_base, const int64_t * S,
+		const uint32_t * idx, const uint64_t * val_of, int4 * segs, uint32_t * seg_off, uint64_t * seg_val)
+{
+	const int64_t n = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
+	const int64_t sg = n / L;
+	const int i = (int) (n % L);
+	if (sg >= nseg)
+		return;
+	int64_t lo = 0, hi = G - 1;
+	while (lo < hi) {
+		const int64_t mid = (lo + hi + 1) >> 1;
+		if (seg_base[mid] <= sg)
+			lo = mid;
+		else
+			hi = mid - 1;
+	}
+	const int64_t g = lo, rf = g_rf[g], u = g_u[g], SE = div_segment_entries(L);
+	const GroupSegments k(u, rf, L);
+	const int64_t j = sg - seg_base[g];
+	const bool rest = j >= k.full;
+	const int64_t pos = rest ? k.dv : j / k.parts * k.np;
+	const int64_t part = rest ? j - k.full : j % k.parts;
+	const int64_t np = rest ? 0 : (k.dv - pos < k.np ? k.dv - pos : k.np);
+	const int64_t nuniq = rest ? k.md : np * L, ncoord = nuniq * rf;
+	const int64_t c0 = part * SE, c1 = c0 + SE < ncoord && (rest || k.parts > 1) ? c0 + SE : ncoord;
+	// segments of the group before this one that continue a lane: all but those at position 0
+	const int64_t at0 = k.full > 0 ? k.parts : 0;
+	const int64_t vi = pos > 0 ? val_base[g] + (j - at0) : -1;
+	if (i == 0) {
+		const int64_t p = g_pkt[g];
+		segs[2 * sg] = make_int4((int) (g_ustart[g] - g_ustart[pk_g0[p]] + pos * L), (int) nuniq, (int) rf,
+				(int) (g_start[g] - pk_j[p] + pos * L * rf));
+		segs[2 * sg + 1] = make_int4((int) c0, (int) c1, (int) vi, rest ? 1 : 0);
+	}
+	uint32_t off = 0;
+	uint64_t val = 0;
+	if (!rest || i < k.md) {
+		const int64_t q0 = seg_start(i, k.dv, k.md), ug = g_ustart[g] + q0;
+		off = (uint32_t) (gl_base[g * L + i] + S[ug + pos] - S[ug]);
+		if (pos > 0)
+			val = val_of[idx[g_start[g] + (q0 + pos - 1) * rf]];
+	}
+	seg_off[sg * L + i] = off;
+	if (vi >= 0)
+		seg_val[vi * L + i] = val;
+}
+
 // ------------------------------------------------------------------ packet reordering
 // DIV_PACKET_REORDERING (div.cpp:377-395, :455-498): every thread's packet groups are
 // stored in ascending order of a median column.  The reference records, per packet, the
@@ -1104,6 +1453,9 @@ int convert_div(Handle & h)
 		set_error(SPMV_ERR_ARG, "DIV-RF: kernel %d unavailable (0, or 2 with vec_len 32)", h.desc.kernel);
 		return SPMV_ERR_ARG;
 	}
+	// nothing asked for, lanes within a warp: the segment decoder
+	if (h.desc.kernel < 0 && L <= 32 && h.desc.block_nnz == 0 && h.desc.stages == 0 && h.desc.ctas_per_sm == 0)
+		h.exec_kernel = 3;
 	// dropped mantissa bits of the lossy mode (reduce_precision, div_kernels_rf.h:467-510)
 	int drop = -1;
 	if (h.desc.div_tolerance > 0) {
@@ -1315,6 +1667,36 @@ int convert_div(Handle & h)
 			u_nb.as<int32_t>(), u_pay.as<uint64_t>(), L, h.d_div);
 	SPMV_CUDA_TRY(cudaGetLastError());
 
+	if (h.exec_kernel == 3) {
+		// segments of the decoder, each lane's place and value at their starts
+		DevBuf cnt3, nval3, base3, vbase3;
+		SPMV_TRY(cnt3.alloc(G * 8, s));
+		SPMV_TRY(nval3.alloc(G * 8, s));
+		SPMV_TRY(base3.alloc((G + 1) * 8, s));
+		SPMV_TRY(vbase3.alloc((G + 1) * 8, s));
+		div_seg_count_kernel<<<(unsigned) ceil_div(G, 256), 256, 0, s>>>(g_u.as<int64_t>(), g_rf.as<int32_t>(), G, L,
+				cnt3.as<int64_t>(), nval3.as<int64_t>());
+		SPMV_CUDA_TRY(cudaGetLastError());
+		SPMV_TRY(scan_exclusive(cnt3.as<int64_t>(), base3.as<int64_t>(), G, s));
+		SPMV_TRY(scan_exclusive(nval3.as<int64_t>(), vbase3.as<int64_t>(), G, s));
+		int64_t nseg = 0, nvals = 0;
+		SPMV_CUDA_TRY(cudaMemcpyAsync(&nseg, base3.as<int64_t>() + G, 8, cudaMemcpyDeviceToHost, s));
+		SPMV_CUDA_TRY(cudaMemcpyAsync(&nvals, vbase3.as<int64_t>() + G, 8, cudaMemcpyDeviceToHost, s));
+		SPMV_CUDA_TRY(cudaStreamSynchronize(s));
+		SPMV_TRY(h.alloc(&h.d_pkt_seg, NP + 1));
+		SPMV_TRY(h.alloc(&h.d_segs, 2 * nseg));
+		SPMV_TRY(h.alloc(&h.d_seg_off, nseg * L));
+		SPMV_TRY(h.alloc(&h.d_seg_val, nvals * L));
+		div_pkt_seg_kernel<<<(unsigned) ceil_div(NP + 1, 256), 256, 0, s>>>(pk_g0.as<int32_t>(), base3.as<int64_t>(), NP,
+				h.d_pkt_seg);
+		SPMV_CUDA_TRY(cudaGetLastError());
+		div_sync_kernel<<<(unsigned) ceil_div(nseg * L, 256), 256, 0, s>>>(base3.as<int64_t>(), vbase3.as<int64_t>(), G, nseg,
+				L, g_u.as<int64_t>(), g_rf.as<int32_t>(), g_ustart.as<int64_t>(), g_start.as<int64_t>(),
+				g_pkt.as<int32_t>(), pk_g0.as<int32_t>(), pk_j.as<int32_t>(), gl_base.as<int64_t>(), S.as<int64_t>(),
+				idx.as<uint32_t>(), val_of.as<uint64_t>(), h.d_segs, h.d_seg_off, h.d_seg_val);
+		SPMV_CUDA_TRY(cudaGetLastError());
+	}
+
 	// 9) packet groups per reference thread (export) and thread byte counts
 	DevBuf th_first, g32, gex2, gbase;
 	SPMV_TRY(th_first.alloc((T + 1) * 8, s));
@@ -1452,6 +1834,31 @@ int launch_div(Handle & h, const double * d_x, double * d_y, cudaStream_t s)
 	if (h.num_split > 0) {
 		zero_rows_kernel<<<(unsigned) ceil_div(h.num_split, 256), 256, 0, s>>>(h.d_split_rows, h.num_split, d_y);
 		SPMV_CUDA_TRY(cudaGetLastError());
+	}
+	if (h.exec_kernel == 3) {
+		DivSegArgs g;
+		g.data = h.d_div;
+		g.pkt_off = h.d_pkt;
+		g.meta = h.d_pkt_meta;
+		g.pkt_seg = h.d_pkt_seg;
+		g.segs = h.d_segs;
+		g.seg_off = h.d_seg_off;
+		g.seg_val = h.d_seg_val;
+		g.end = h.d_div + h.div_bytes;
+		g.x = d_x;
+		g.y = d_y;
+		void (*kern)(DivSegArgs) = nullptr;
+		switch (h.desc.vec_len) {
+		case 1: kern = div_segment_kernel<1>; break;
+		case 2: kern = div_segment_kernel<2>; break;
+		case 4: kern = div_segment_kernel<4>; break;
+		case 8: kern = div_segment_kernel<8>; break;
+		case 16: kern = div_segment_kernel<16>; break;
+		default: kern = div_segment_kernel<32>; break;
+		}
+		kern<<<(unsigned) h.num_packets, DIVS_THREADS, 0, s>>>(g);
+		SPMV_CUDA_TRY(cudaGetLastError());
+		return SPMV_OK;
 	}
 	DivArgs a;
 	a.data = h.d_div;

@@ -158,6 +158,12 @@ struct Handle {
 	uint8_t * d_div = nullptr;
 	int64_t * d_pkt = nullptr;          // packet byte offsets [num_packets+1]
 	int4 * d_pkt_meta = nullptr;        // per packet: {y row start, y row end, flags, 0}
+	// segment decoder (exec_kernel 3): packets' segments, their descriptors, and each lane's
+	// payload byte and value at their starts
+	int32_t * d_pkt_seg = nullptr;
+	int4 * d_segs = nullptr;
+	uint32_t * d_seg_off = nullptr;
+	uint64_t * d_seg_val = nullptr;
 	int64_t * d_groups = nullptr;       // per-thread group offsets (concatenated)
 	int64_t num_group_entries = 0;
 	int64_t * d_thread_bytes = nullptr;
