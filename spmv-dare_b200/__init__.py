@@ -89,6 +89,20 @@ def _is_cuda_tensor(a):
 
 CUDA_STREAM_LEGACY = 1   # cudaStreamLegacy: torch's default stream reports handle 0
 
+_torch = None            # the torch module and its raw current-stream lookup, once a CUDA tensor is seen
+_current_raw_stream = None
+
+
+def _use_torch():
+    global _torch, _current_raw_stream
+    if _torch is None:
+        import torch
+
+        _current_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
+            lambda device: torch.cuda.current_stream(device).cuda_stream)
+        _torch = torch
+    return _torch
+
 
 def _torch_stream(device, stream=None):
     """Raw cudaStream_t of `stream` (a torch.cuda.Stream or raw handle) or of torch's current
@@ -142,21 +156,24 @@ class Matrix_Format:
         if self._h is None:
             raise SpmvError(_capi.SPMV_ERR_ARG, "matrix already destroyed")
         self.num_loops += 1
-        lib = library()
+        lib = _capi._lib or library()
         if _is_cuda_tensor(x):
-            import torch
-
+            torch = _torch or _use_torch()
+            xt = x.dtype
             if y is None:
-                y = torch.empty(self.m, dtype=x.dtype, device=x.device)
+                y = torch.empty(self.m, dtype=xt, device=x.device)
             if not (x.is_contiguous() and y.is_contiguous()):
                 raise ValueError("x and y must be contiguous")
             if x.numel() < self.n or y.numel() < self.m:
                 raise ValueError(f"x needs {self.n} and y {self.m} elements")
-            s = _torch_stream(x.device, stream)
-            if x.dtype == torch.float32:
+            if stream is None:
+                s = _current_raw_stream(x.get_device()) or CUDA_STREAM_LEGACY
+            else:
+                s = _torch_stream(x.device, stream)
+            if xt is torch.float32:
                 st = lib.spmv_run_device_f32(self._h, x.data_ptr(), y.data_ptr(), s)
             else:
-                if x.dtype != torch.float64 or y.dtype != torch.float64:
+                if xt is not torch.float64 or y.dtype is not torch.float64:
                     raise TypeError("x and y must both be float64 (or both float32 for the FP32 variant)")
                 st = lib.spmv_run_device(self._h, x.data_ptr(), y.data_ptr(), s)
             if st:

@@ -3,6 +3,7 @@
 #include <string.h>
 
 #include <chrono>
+#include <mutex>
 #include <string>
 
 #include "hostcopy.h"
@@ -32,6 +33,49 @@ void clear_error()
 {
 	g_status = SPMV_OK;
 	g_msg[0] = 0;
+}
+
+// Pools are made on first use and kept for the process.
+cudaError_t pool_alloc(void ** p, size_t bytes, Pool kind, cudaStream_t s)
+{
+	constexpr int MOST = 64;
+	static std::mutex lock;
+	static cudaMemPool_t pools[MOST][2];
+	int dev = 0;
+	cudaError_t e = cudaGetDevice(&dev);
+	if (e != cudaSuccess || dev >= MOST)
+		return e != cudaSuccess ? e : cudaErrorInvalidDevice;
+	cudaMemPool_t both[2];
+	{
+		std::lock_guard<std::mutex> hold(lock);
+		for (int k = 0; k < 2; k++) {
+			if (!pools[dev][k]) {
+				cudaMemPoolProps props{};
+				props.allocType = cudaMemAllocationTypePinned;
+				props.location.type = cudaMemLocationTypeDevice;
+				props.location.id = dev;
+				unsigned long long keep = POOL_KEEP_BYTES;
+				cudaMemPool_t made = nullptr;
+				if ((e = cudaMemPoolCreate(&made, &props)) != cudaSuccess)
+					return e;
+				if ((e = cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) {
+					cudaMemPoolDestroy(made);
+					return e;
+				}
+				pools[dev][k] = made;
+			}
+			both[k] = pools[dev][k];
+		}
+	}
+	e = cudaMallocFromPoolAsync(p, bytes, both[(int) kind], s);
+	if (e == cudaErrorMemoryAllocation) {
+		cudaGetLastError();
+		cudaDeviceSynchronize();
+		for (cudaMemPool_t q : both)
+			cudaMemPoolTrimTo(q, 0);
+		e = cudaMallocFromPoolAsync(p, bytes, both[(int) kind], s);
+	}
+	return e;
 }
 
 static const char * kNames[SPMV_NUM_FORMATS] = {
@@ -139,14 +183,21 @@ static int check_desc(const spmv_format_desc & d)
 // Releases every device resource of a handle (the Handle object itself is owned by the caller).
 static void release_handle(Handle & h)
 {
-	if (h.stream)
-		cudaStreamSynchronize(h.stream);
-	for (void * p : h.allocations)
-		cudaFree(p);
+	if (!h.stream)
+		return;                    // no device yet, so nothing allocated
+	// the caller's SpMVs may run on any stream: the memory goes back once all work is done
+	int cur = h.device;
+	cudaGetDevice(&cur);
+	if (cur != h.device)
+		cudaSetDevice(h.device);
+	cudaDeviceSynchronize();
+	for (const Handle::Allocation & a : h.allocations)
+		a.pooled ? cudaFreeAsync(a.p, h.stream) : cudaFree(a.p);
 	h.allocations.clear();
-	if (h.stream)
-		cudaStreamDestroy(h.stream);
+	cudaStreamDestroy(h.stream);
 	h.stream = nullptr;
+	if (cur != h.device)
+		cudaSetDevice(cur);
 }
 
 // Reference mem_footprint of each format (bytes).

@@ -182,13 +182,17 @@ struct Handle {
 
 	bool convert_only = false;          // a batch's matrix: no execution schedule of its own
 
-	std::vector<void *> allocations;    // everything above, freed by destroy
+	struct Allocation {
+		void * p;
+		bool pooled;
+	};
+	std::vector<Allocation> allocations;    // everything above, freed by destroy
 	double mem_footprint = 0;
 	double csr_mem_footprint = 0;
 	int64_t stored_elems = 0;
 	int64_t device_bytes = 0;
 	double convert_ms = 0;
-	double alloc_ms = 0;        // host time inside cudaMalloc during the conversion
+	double alloc_ms = 0;        // host time inside allocations during the conversion
 	double copy_in_ms = 0;      // the CSR arrays' copy to the device (until it completed)
 	int64_t x_lo = 0, x_hi = -1;  // span of the format's columns above 0 (inclusive; empty if hi < lo)
 	int64_t x_col0 = 0;           // column 0 occurs (SELL-C-sigma pads with it)
@@ -200,14 +204,15 @@ struct Handle {
 	{
 		size_t bytes = (size_t) (count > 0 ? count : 1) * sizeof(T);
 		const auto t0 = std::chrono::steady_clock::now();
-		cudaError_t e = cudaMalloc((void **) p, bytes);
+		const bool pooled = bytes <= POOL_MOST_BYTES;
+		cudaError_t e = pooled ? pool_alloc((void **) p, bytes, Pool::HANDLE, stream) : cudaMalloc((void **) p, bytes);
 		alloc_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
 		if (e != cudaSuccess) {
 			*p = nullptr;
-			set_error(SPMV_ERR_NOMEM, "cudaMalloc(%zu) failed: %s", bytes, cudaGetErrorString(e));
+			set_error(SPMV_ERR_NOMEM, "device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
 			return SPMV_ERR_NOMEM;
 		}
-		allocations.push_back((void *) *p);
+		allocations.push_back({(void *) *p, pooled});
 		device_bytes += (int64_t) bytes;
 		return SPMV_OK;
 	}

@@ -76,7 +76,7 @@ struct DevBuf {
 	int alloc(size_t bytes, cudaStream_t stream)
 	{
 		s = stream;
-		cudaError_t e = cudaMallocAsync(&p, bytes ? bytes : 16, stream);
+		cudaError_t e = pool_alloc(&p, bytes ? bytes : 16, Pool::SCRATCH, stream);
 		if (e != cudaSuccess) {
 			p = nullptr;
 			set_error(SPMV_ERR_NOMEM, "scratch allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
