@@ -1075,6 +1075,7 @@ template <int L>
 __global__ void __launch_bounds__(DIVS_THREADS, 6) div_segment_kernel(DivSegArgs a)
 {
 	__shared__ double ys[DEC_MAX_ROWS];
+	release_next();
 	const int64_t p = blockIdx.x;
 	const int t = threadIdx.x & 31, l = t & (L - 1);
 	const uint8_t * h = a.data + a.pkt_off[p];
@@ -1113,6 +1114,7 @@ __global__ void __launch_bounds__(DIVS_THREADS, 6) div_segment_kernel(DivSegArgs
 			prefetch_l1(q + (o < bytes ? o : bytes - 1), a.end);
 	};
 	fetch(s);
+	wait_previous();
 	for (int r = threadIdx.x; r < nrows && r < DEC_MAX_ROWS; r += blockDim.x)
 		ys[r] = 0.0;
 	__syncthreads();
@@ -1139,7 +1141,7 @@ __global__ void __launch_bounds__(DIVS_THREADS, 6) div_segment_kernel(DivSegArgs
 				at += (uint32_t) __shfl_sync(0xffffffffu, ends, 32 - L + l);
 				if (u + t < nuniq) {
 					coords.get(coord0 + u + t, r, col);
-					xx = __ldg(x + col);
+					xx = load_x(x + col);
 				}
 			};
 			ahead(0, code, w, row, xv);
@@ -1179,7 +1181,7 @@ __global__ void __launch_bounds__(DIVS_THREADS, 6) div_segment_kernel(DivSegArgs
 				double xe = 0.0;
 				if (on) {
 					coords.get((int64_t) coord0 + u0 * rf + e, row, col);
-					xe = __ldg(x + col);
+					xe = load_x(x + col);
 				}
 				// the thread that holds the coordinate's value: e / rf in an incomplete position,
 				// else lane e % L of position e / (L rf)
@@ -1856,8 +1858,7 @@ int launch_div(Handle & h, const double * d_x, double * d_y, cudaStream_t s)
 		case 16: kern = div_segment_kernel<16>; break;
 		default: kern = div_segment_kernel<32>; break;
 		}
-		kern<<<(unsigned) h.num_packets, DIVS_THREADS, 0, s>>>(g);
-		SPMV_CUDA_TRY(cudaGetLastError());
+		SPMV_CUDA_TRY(launch_overlapped(kern, (unsigned) h.num_packets, DIVS_THREADS, 0, s, g));
 		return SPMV_OK;
 	}
 	DivArgs a;

@@ -259,6 +259,7 @@ __global__ void __launch_bounds__(512) ws_f32_kernel(F32WsArgs a)
 	extern __shared__ __align__(128) uint8_t smem[];
 	__shared__ StagedBlock sdesc[8];
 	__shared__ int4 spack[8];
+	release_next();
 	const int S = a.stages;
 	uint64_t * full = reinterpret_cast<uint64_t *>(smem + (size_t) S * a.stage_bytes);
 	uint64_t * prod = full + S;
@@ -278,6 +279,7 @@ __global__ void __launch_bounds__(512) ws_f32_kernel(F32WsArgs a)
 	if ((int) threadIdx.x < ng) {
 		// ---- gather warps: x of every staged entry, WS_GATHER_SLOTS loads in flight per thread
 		const int gt = threadIdx.x;
+		wait_previous();                                   // x from here on
 		for (int64_t b = b_begin; b < b_end; b++) {
 			const bool ok = mbar_wait_bounded(&full[s], parity, a.wait_budget);
 			if (named_bar_or(2, ng, !ok)) {                // the gather warps leave together
@@ -302,7 +304,7 @@ __global__ void __launch_bounds__(512) ws_f32_kernel(F32WsArgs a)
 					for (int k = 0; k < WS_GATHER_SLOTS; k++) {
 						const int e = rb + gt + k * ng;
 						if (e < d.elems)
-							xv[k] = __ldg(a.x + packed_col(words, e, pi.z, pi.y));
+							xv[k] = load_x(a.x + packed_col(words, e, pi.z, pi.y));
 					}
 					named_bar_sync(2, ng);
 					#pragma unroll
@@ -323,7 +325,7 @@ __global__ void __launch_bounds__(512) ws_f32_kernel(F32WsArgs a)
 					for (int k = 0; k < WS_GATHER_SLOTS; k++) {
 						const int e = e0 + k * ng;
 						if (e < d.elems)
-							xv[k] = __ldg(a.x + sc[off + e]);
+							xv[k] = load_x(a.x + sc[off + e]);
 					}
 					#pragma unroll
 					for (int k = 0; k < WS_GATHER_SLOTS; k++) {
@@ -360,6 +362,7 @@ __global__ void __launch_bounds__(512) ws_f32_kernel(F32WsArgs a)
 				}
 			}
 		}
+	wait_previous();                                       // y from here on
 	named_bar_sync(1, nr);
 	float ls = 0.0f, lc = 0.0f;      // running Dot2 pair of a long row across its chunks
 	for (int64_t b = b_begin; b < b_end; b++) {
@@ -1370,10 +1373,9 @@ int launch_spmv_f32(Handle & h, const float * d_x, float * d_y, cudaStream_t s)
 		w.pcols = h.d_pcols;
 		w.rassign = h.d_rassign;
 		if (h.d_pcols)
-			ws_f32_kernel<true><<<h.grid, h.threads, h.smem_bytes, s>>>(w);
+			SPMV_CUDA_TRY(launch_overlapped(ws_f32_kernel<true>, (unsigned) h.grid, (unsigned) h.threads, h.smem_bytes, s, w));
 		else
-			ws_f32_kernel<false><<<h.grid, h.threads, h.smem_bytes, s>>>(w);
-		SPMV_CUDA_TRY(cudaGetLastError());
+			SPMV_CUDA_TRY(launch_overlapped(ws_f32_kernel<false>, (unsigned) h.grid, (unsigned) h.threads, h.smem_bytes, s, w));
 		return SPMV_OK;
 	}
 	F32Args a{};

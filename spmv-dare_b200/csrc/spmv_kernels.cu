@@ -873,6 +873,7 @@ __global__ void __launch_bounds__(STAGED_MAX_THREADS) ws_kernel(StagedArgs a)
 	extern __shared__ __align__(128) uint8_t smem[];
 	__shared__ StagedBlock sdesc[8];
 	__shared__ int4 spack[8];
+	release_next();
 	const int S = a.stages;
 	uint64_t * full = reinterpret_cast<uint64_t *>(smem + (size_t) S * a.stage_bytes);
 	uint64_t * prod = full + S;
@@ -892,6 +893,7 @@ __global__ void __launch_bounds__(STAGED_MAX_THREADS) ws_kernel(StagedArgs a)
 	if ((int) threadIdx.x < ng) {
 		// ---- gather warps
 		const int gt = threadIdx.x;
+		wait_previous();                                   // x from here on
 		for (int64_t b = b_begin; b < b_end; b++) {
 			const bool ok = mbar_wait_bounded(&full[s], parity, a.wait_budget);
 			if (named_bar_or(2, ng, !ok)) {                // the gather warps leave together
@@ -921,7 +923,7 @@ __global__ void __launch_bounds__(STAGED_MAX_THREADS) ws_kernel(StagedArgs a)
 					for (int k = 0; k < WS_GATHER_SLOTS; k++) {
 						const int e = e0 + k * ng;
 						if (e < d.elems)
-							xv[k] = ldg(a.x + (PK ? packed_col64(words, e, pi.z, pi.y) : sc[off + e]));
+							xv[k] = load_x(a.x + (PK ? packed_col64(words, e, pi.z, pi.y) : sc[off + e]));
 					}
 					if (A != Arith::SEQ_SPLIT)
 						named_bar_sync(2, ng);
@@ -966,6 +968,7 @@ __global__ void __launch_bounds__(STAGED_MAX_THREADS) ws_kernel(StagedArgs a)
 				}
 			}
 		}
+	wait_previous();                                       // y from here on
 	named_bar_sync(1, nr);
 	double acc = 0.0;          // running state of a long unit across its chunk blocks
 	double ln[L];
@@ -1607,6 +1610,10 @@ int launch_spmv(Handle & h, const double * d_x, double * d_y, cudaStream_t s)
 		a.stage_bytes = ws_stage_layout(fmt, a.cap_al, true, &a.cols_off);
 		a.row_threads = h.row_threads;
 		a.ranges = h.d_cta_ranges;
+	}
+	if (h.exec_kernel == 4 || h.exec_kernel == 8) {
+		SPMV_CUDA_TRY(launch_overlapped(kern, (unsigned) h.grid, (unsigned) h.threads, h.smem_bytes, s, a));
+		return SPMV_OK;
 	}
 	kern<<<h.grid, h.threads, h.smem_bytes, s>>>(a);
 	SPMV_CUDA_TRY(cudaGetLastError());

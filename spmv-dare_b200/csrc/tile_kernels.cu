@@ -361,6 +361,7 @@ __device__ void long_unit(const TileArgs & a, const LongUnit & u, int lane, type
 		}
 	};
 	load(0);
+	wait_previous();
 	RowSum<S> acc;
 	T s = T(0);
 	for (int e0 = 0; e0 < u.n; e0 += LONG_STEP) {
@@ -368,7 +369,7 @@ __device__ void long_unit(const TileArgs & a, const LongUnit & u, int lane, type
 		#pragma unroll
 		for (int i = 0; i < PER; i++) {
 			const int e = e0 + i * 32 + lane;
-			xv[i] = e < u.n ? __ldg(x + c[i]) : T(0);
+			xv[i] = e < u.n ? load_x(x + c[i]) : T(0);
 			v[i] = vn[i];
 		}
 		load(e0 + LONG_STEP);
@@ -467,6 +468,7 @@ __global__ void __launch_bounds__(TILE_THREADS, MINB) tile_kernel(TileArgs a)
 	const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 	const int cta = (int) blockIdx.x;
 	int w;
+	release_next();
 	if (cta < a.nlong) {
 		if (wid == 0) {
 			long_unit<S>(a, a.longs[cta], lane, xs[0][0], xs[0][1]);
@@ -476,12 +478,12 @@ __global__ void __launch_bounds__(TILE_THREADS, MINB) tile_kernel(TileArgs a)
 	} else {
 		w = cta * TILE_WARPS + wid - a.nlong;
 	}
-	if (w >= a.nranges)
-		return;
-	const int4 range = __ldg(a.ranges + w);
+	const int4 range = w < a.nranges ? __ldg(a.ranges + w) : make_int4(0, 0, 0, 0);
 	int sl = range.x;
-	if (sl >= range.y)
+	if (sl >= range.y) {
+		wait_previous();
 		return;
+	}
 	const T * __restrict__ x = static_cast<const T *>(a.x);
 	const T * __restrict__ vals = static_cast<const T *>(a.vals);
 	T * __restrict__ y = static_cast<T *>(a.y);
@@ -504,14 +506,14 @@ __global__ void __launch_bounds__(TILE_THREADS, MINB) tile_kernel(TileArgs a)
 	auto gather = [&](uint32_t buf, int tw) {
 		if constexpr (STAGED) {
 			if (col < tw) {
-				X[0] = __ldg(x + c0.x);
-				X[1] = __ldg(x + c0.y);
-				X[2] = __ldg(x + c0.z);
-				X[3] = __ldg(x + c0.w);
-				X[4] = __ldg(x + c1.x);
-				X[5] = __ldg(x + c1.y);
-				X[6] = __ldg(x + c1.z);
-				X[7] = __ldg(x + c1.w);
+				X[0] = load_x(x + c0.x);
+				X[1] = load_x(x + c0.y);
+				X[2] = load_x(x + c0.z);
+				X[3] = load_x(x + c0.w);
+				X[4] = load_x(x + c1.x);
+				X[5] = load_x(x + c1.y);
+				X[6] = load_x(x + c1.z);
+				X[7] = load_x(x + c1.w);
 			}
 			return;
 		}
@@ -546,6 +548,7 @@ __global__ void __launch_bounds__(TILE_THREADS, MINB) tile_kernel(TileArgs a)
 	load_values(vals + t0, q & 15, lane, v[0]);
 	int n = __ldg(a.slot_cnt + (int64_t) sl * 32 + lane), row = __ldg(a.slot_row + (int64_t) sl * 32 + lane);
 	const uint32_t d1 = cu.next(a.sptr);
+	wait_previous();
 	gather(0, q & 15);
 	if constexpr (STAGED)
 		store_x(0, q & 15);
@@ -1006,8 +1009,8 @@ int launch_tiles(const TilePlan & p, int format, int lanes, const void * x, void
 	a.nranges = (int) p.nranges;
 	a.longs = p.longs;
 	a.nlong = (int) p.nlong;
-	tile_fn(format, lanes, p.f32, p.mixed, p.wide, p.staged)<<<(unsigned) p.grid, TILE_THREADS, 0, s>>>(a);
-	SPMV_CUDA_TRY(cudaGetLastError());
+	SPMV_CUDA_TRY(launch_overlapped(tile_fn(format, lanes, p.f32, p.mixed, p.wide, p.staged), (unsigned) p.grid, TILE_THREADS, 0,
+			s, a));
 	return SPMV_OK;
 }
 
