@@ -508,9 +508,13 @@ TileSource tile_source(const Handle & h)
 	if (h.desc.format == SPMV_FMT_SELL_C_S) {
 		t.P = h.d_sptr32;
 		t.V = h.desc.sellcs_c;
+		t.rp = h.d_rp;
+		t.pad_col = 0;                  // sellcs_format.c:137-200
 	} else if (h.desc.format == SPMV_FMT_SELL || h.desc.format == SPMV_FMT_SELL_SORTED) {
 		t.P = h.d_rcp;
 		t.V = h.desc.vec_len;
+		t.rp = h.d_rp;
+		t.pad_col = PAD_OWN;            // sell.cpp:165, 182-191
 	}
 	t.m = h.m;
 	t.split = h.desc.format == SPMV_FMT_CSR_NAIVE;

@@ -22,8 +22,14 @@ struct TileSource {
 	int64_t m;                   // rows
 	int64_t entries;             // stored entries
 	bool split;                  // csr_naive arithmetic: product and sum rounded separately
+	// Padded slices: the CSR row_ptr (null: rows have no padding), and the column that pads a
+	// row, PAD_OWN for the row's own last one.
+	const int32_t * rp;
+	int32_t pad_col;
 	int64_t x_off, y_off;        // batches: offsets into the concatenated x and y
 };
+
+constexpr int32_t PAD_OWN = -1, PAD_SPLIT = -2;
 
 // A row summed by a whole warp from the format's own arrays.
 struct LongUnit {
@@ -34,17 +40,19 @@ struct LongUnit {
 	int32_t x_off;
 	int32_t split;               // csr_naive arithmetic (batches)
 	int32_t row;                 // y index
+	int32_t padded, pad_col;     // the row ends in padding; its column (PAD_OWN: that of the last entry)
 };
 
 struct TilePlan {
 	bool built = false;
+	int32_t pad_col = PAD_OWN;
 	bool f32 = false, mixed = false, wide = false, staged = false;
 	int32_t * sptr = nullptr;
 	int32_t * tcols = nullptr;
 	void * vals = nullptr;
 	int32_t * slot_row = nullptr;
 	int32_t * slot_cnt = nullptr;
-	uint8_t * split = nullptr;
+	int32_t * pad = nullptr;     // MIXED batches: a slice's pad column, PAD_OWN or PAD_SPLIT
 	int4 * ranges = nullptr;
 	LongUnit * longs = nullptr;
 	int64_t nranges = 0, nlong = 0, grid = 0;

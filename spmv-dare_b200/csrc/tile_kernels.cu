@@ -74,11 +74,12 @@ struct RowSum<Sum::NAIVE> : SplitSum {};
 
 struct FusedSum {                               // one fused multiply-add per slice column
 	using T = double;
-	double s = 0.0;
+	double s = 0.0, last = 0.0;                 // and the x of the last one
 	template <int J, bool FULL>
 	__device__ __forceinline__ void step(int k, int n, double v, double x)
 	{
 		s = __fma_rn(FULL || k < n ? v : -0.0, FULL || k < n ? x : 1.0, s);
+		last = FULL || k < n ? x : last;
 	}
 	__device__ __forceinline__ double total(int) const { return s; }
 };
@@ -328,9 +329,10 @@ struct TileArgs {
 	const void * vals;
 	const int32_t * slot_row; // y index of each slot, -1: none
 	const int32_t * slot_cnt; // entries of each slot
-	const uint8_t * split;    // MIXED: the slice multiplies and adds separately
+	const int32_t * pad;      // MIXED: each slice's pad column or arithmetic
 	const void * x;
 	void * y;
+	int32_t pad_col;          // column that ends a padded row, PAD_OWN: its last one's
 	const int4 * ranges;      // per warp: first slice, end, first entry, end of the first slice
 	int nranges;
 	const LongUnit * longs;
@@ -419,12 +421,22 @@ __device__ void long_unit(const TileArgs & a, const LongUnit & u, int lane, type
 		if (lane == 0)
 			y[u.row] = acc.total(u.n);
 	} else {
-		if (lane == 0)
+		if (lane == 0) {
+			if (!split && u.padded)
+				s = __fma_rn(0.0, load_x(x + (u.pad_col == PAD_OWN ? u.cols[at(u.n - 1)] : u.pad_col)), s);
 			y[u.row] = s;
+		}
 	}
 }
 
 // ------------------------------------------------------------------ the kernel
+// A slot's count; PADDED: the row's slice is wider than the row.  Any number of padding entries
+// (value 0, one column) adds what one does: 0 * x is a zero, or NaN, and adding it again changes
+// nothing.  So padding is not stored: one fused multiply-add with the pad column's x ends the row.
+// SELL on 2M rows of 26 +- 3 in slices of 4: 137 -> 132 us, 500,000 rows of 50 +- 35 in slices of 8:
+// 169 (kernel 4) -> 76, the 48-matrix batch 113 -> 98.
+constexpr int PADDED = 1 << 30, COUNT = PADDED - 1;
+
 // The tiles of a range in order.  next() gives the tile's width (0 .. 8) with TILE_LAST on the
 // last one of a slice, and 0 past the end of the range; t0 is the tile's first entry.
 constexpr uint32_t TILE_LAST = 16, TILE_BITS = 5, TILE_MASK = 31;
@@ -560,8 +572,11 @@ __global__ void __launch_bounds__(TILE_THREADS, MINB) tile_kernel(TileArgs a)
 		rown = __ldg(a.slot_row + (int64_t) (sl + 1) * 32 + lane);
 	}
 	RowSum<S> acc;
-	if constexpr (S == Sum::MIXED)
-		acc.split = a.split[sl] != 0;
+	int pad = a.pad_col;
+	if constexpr (S == Sum::MIXED) {
+		pad = a.pad[sl];
+		acc.split = pad == PAD_SPLIT;
+	}
 	uint32_t buf = 0;
 	// one tile, its values in vt; the next tile's go to vn.  Returns false after the last.
 	auto tile = [&](T (&vt)[8], T (&vn)[8]) -> bool {
@@ -576,8 +591,9 @@ __global__ void __launch_bounds__(TILE_THREADS, MINB) tile_kernel(TileArgs a)
 			asm volatile("cp.async.wait_group 1;" ::: "memory");
 		__syncwarp();
 		const int k0 = (t0 - b) >> 5;
-		const bool full = __all_sync(0xffffffffu, k0 + 8 <= (n & WHOLE));
-		add_tile<S>(acc, full, k0, n, vt, xrow + buf);
+		const int cnt = n & COUNT;
+		const bool full = __all_sync(0xffffffffu, k0 + 8 <= (cnt & WHOLE));
+		add_tile<S>(acc, full, k0, cnt, vt, xrow + buf);
 		if (!AHEAD)
 			load_values(vals + t1, q >> TILE_BITS & 15, lane, vn);
 		if constexpr (STAGED)
@@ -588,14 +604,19 @@ __global__ void __launch_bounds__(TILE_THREADS, MINB) tile_kernel(TileArgs a)
 		t0 = t1;
 		buf ^= BUF;
 		if (last) {
+			if constexpr (S == Sum::FMA || S == Sum::MIXED)
+				if (n & PADDED)
+					acc.s = __fma_rn(0.0, pad == PAD_OWN ? acc.last : load_x(x + pad), acc.s);
 			if (row >= 0)
 				y[row] = acc.total(n);
 			if ((q & TILE_MASK) == 0)
 				return false;
 			acc = RowSum<S>();
 			sl++;
-			if constexpr (S == Sum::MIXED)
-				acc.split = a.split[sl] != 0;
+			if constexpr (S == Sum::MIXED) {
+				pad = a.pad[sl];
+				acc.split = pad == PAD_SPLIT;
+			}
 			b = t1;
 			n = nn;
 			row = rown;
@@ -616,8 +637,9 @@ __global__ void __launch_bounds__(TILE_THREADS, MINB) tile_kernel(TileArgs a)
 }
 
 // ------------------------------------------------------------------ building the layout
-// Entries of row i of a source: start and stride in its arrays, count.
-__device__ __forceinline__ void source_row(const TileSource & s, int64_t i, int64_t & start, int & stride, int & cnt)
+// Entries of row i of a source: start and stride in its arrays, count, and whether padding
+// follows them (a row that is all padding keeps one entry of it).
+__device__ __forceinline__ bool source_row(const TileSource & s, int64_t i, int64_t & start, int & stride, int & cnt)
 {
 	if (s.V == 1) {
 		start = s.P[i];
@@ -629,6 +651,16 @@ __device__ __forceinline__ void source_row(const TileSource & s, int64_t i, int6
 		stride = s.V;
 		cnt = (int) (((int64_t) s.P[sl + 1] - p) / s.V);
 	}
+	if (!s.rp)
+		return false;
+	const int64_t r = s.ymap ? s.ymap[i] : i;
+	const int len = s.rp[r + 1] - s.rp[r];
+	if (len == 0)
+		cnt = cnt > 0 ? 1 : 0;
+	const bool padded = len > 0 && len < cnt;
+	if (padded)
+		cnt = len;
+	return padded;
 }
 
 // One CTA per window: its rows sorted by count (descending, stable; long rows and the places
@@ -676,7 +708,9 @@ __global__ void __launch_bounds__(TILE_WINDOW / 2) tile_sort_kernel(TileSource s
 		const int64_t slot = slot0 + base + i;
 		slot_src[slot] = rank == MOST ? -1 : (int32_t) r;
 		slot_row[slot] = rank == MOST ? -1 : (int32_t) (s.y_off + (s.ymap ? s.ymap[r] : r));
-		slot_cnt[slot] = cnt;
+		int64_t start;
+		int stride, own;
+		slot_cnt[slot] = rank != MOST && source_row(s, r, start, stride, own) ? cnt | PADDED : cnt;
 		if (i % 32 == 0)
 			width[slot / 32] = (int64_t) cnt * 32;
 	}
@@ -713,7 +747,7 @@ __global__ void tile_sptr_kernel(const int64_t * in, int64_t n, int32_t * out)
 // One warp per slice, a lane per row: the entries into the tiled layout.
 template <typename T>
 __global__ void tile_fill_kernel(TileSource s, int64_t slice0, int64_t nslices, const int32_t * slot_src,
-		const int32_t * sptr, int32_t * tcols, T * tvals, uint8_t * split)
+		const int32_t * sptr, int32_t * tcols, T * tvals, int32_t * pad_of)
 {
 	const int64_t i = ((int64_t) blockIdx.x * blockDim.x + threadIdx.x) >> 5;
 	const int r = threadIdx.x & 31;
@@ -727,8 +761,8 @@ __global__ void tile_fill_kernel(TileSource s, int64_t slice0, int64_t nslices, 
 	int stride = 1, cnt = 0;
 	if (src >= 0)
 		source_row(s, src, start, stride, cnt);
-	if (split && r == 0)
-		split[sl] = s.split;
+	if (pad_of && r == 0)
+		pad_of[sl] = s.split ? PAD_SPLIT : s.pad_col == PAD_OWN ? PAD_OWN : (int32_t) (s.pad_col + s.x_off);
 	int32_t pad = cnt > 0 ? s.cols[start] : 0;      // columns of the padding: read, never summed
 	for (int k8 = 0; k8 < W; k8 += 8) {
 		const int tw = W - k8 < 8 ? W - k8 : 8;
@@ -806,10 +840,12 @@ __global__ void long_units_kernel(TileSource s, const T * vals, int long_min, in
 		return;
 	int64_t start;
 	int stride, cnt;
-	source_row(s, i, start, stride, cnt);
+	const bool padded = source_row(s, i, start, stride, cnt);
 	if (cnt < long_min)
 		return;
 	LongUnit u;
+	u.padded = padded;
+	u.pad_col = s.pad_col;
 	u.cols = s.cols + start;
 	u.vals = vals + start;
 	u.n = cnt;
@@ -933,7 +969,7 @@ int build_tiles(TilePlan & p, const std::vector<TileSource> & src, bool f32, boo
 	SPMV_TRY(alloc((void **) &p.tcols, total * sizeof(int32_t)));
 	SPMV_TRY(alloc((void **) &p.vals, total * vs));
 	if (mixed)
-		SPMV_TRY(alloc((void **) &p.split, ns));
+		SPMV_TRY(alloc((void **) &p.pad, ns * sizeof(int32_t)));
 	SPMV_TRY(alloc((void **) &p.longs, nlong * sizeof(LongUnit)));
 	tile_sptr_kernel<<<(unsigned) ceil_div(ns + 1, 256), 256, 0, s>>>(sptr64.as<int64_t>(), ns + 1, p.sptr);
 	SPMV_CUDA_TRY(cudaGetLastError());
@@ -945,12 +981,12 @@ int build_tiles(TilePlan & p, const std::vector<TileSource> & src, bool f32, boo
 		const unsigned gl = (unsigned) ceil_div(src[i].m, 256);
 		if (f32) {
 			tile_fill_kernel<float><<<g, 256, 0, s>>>(src[i], slot0[i] / 32, n, d_src.as<int32_t>(), p.sptr, p.tcols,
-					(float *) p.vals, p.split);
+					(float *) p.vals, p.pad);
 			if (nlong > 0)
 				long_units_kernel<float><<<gl, 256, 0, s>>>(src[i], src[i].vals_f, long_min[i], cnt.as<int>() + 1, p.longs);
 		} else {
 			tile_fill_kernel<double><<<g, 256, 0, s>>>(src[i], slot0[i] / 32, n, d_src.as<int32_t>(), p.sptr, p.tcols,
-					(double *) p.vals, p.split);
+					(double *) p.vals, p.pad);
 			if (nlong > 0)
 				long_units_kernel<double><<<gl, 256, 0, s>>>(src[i], src[i].vals, long_min[i], cnt.as<int>() + 1, p.longs);
 		}
@@ -988,6 +1024,7 @@ int build_tiles(TilePlan & p, const std::vector<TileSource> & src, bool f32, boo
 		p.grid = nlong;
 	p.f32 = f32;
 	p.mixed = mixed;
+	p.pad_col = src[0].pad_col;
 	p.built = true;
 	return SPMV_OK;
 }
@@ -1002,7 +1039,8 @@ int launch_tiles(const TilePlan & p, int format, int lanes, const void * x, void
 	a.vals = p.vals;
 	a.slot_row = p.slot_row;
 	a.slot_cnt = p.slot_cnt;
-	a.split = p.split;
+	a.pad = p.pad;
+	a.pad_col = p.pad_col;
 	a.x = x;
 	a.y = y;
 	a.ranges = p.ranges;
