@@ -985,16 +985,36 @@ __global__ void __launch_bounds__(DIVW_WARPS * 32, MINB) div_warp_kernel(DivArgs
 // What bounds it: the L1 pipe (x is read in value order, a line an entry; shared FP64 additions
 // are compare-and-swap loops, about 40 us of 20 M entries) and instruction issue (some 180 a 32
 // entries); DRAM is 9% busy.  Measured in a loop over three matrices, before and now: 4 lanes,
-// 20 M distinct values 244 -> 203 us; 8 M entries of 300 values 454 -> 98 us with 32 lanes (groups
+// 20 M distinct values 244 -> 193 us; 8 M entries of 300 values 454 -> 91 us with 32 lanes (groups
 // of few values left most lanes of the warp decoder idle) and 2,286 -> 91 with 4 (one thread
 // walked a value's coordinates); 32 lanes, distinct values, 4,096-value packets 243 -> 200.
 // Tried: no lookahead 385, lines asked of L1 a segment ahead 303, and the next step's payload
 // and x loads under way 203-211; CTAs of 256 threads 235, of 512 285 (packets of some 5,000
 // entries are their unit of balance); row sums a warp 236; segments of 512 entries 242.
-constexpr int DIVS_THREADS = 128;
+//
+// Row sums: a packet has 2 to 32 for each row, as many as the shared array holds, and
+// neighbouring threads add to different ones.  In a packet of a few long rows the threads of a
+// warp otherwise add to one word in turn: 2.4 M entries, rows of up to 2,000, 147 us with one
+// sum a row, 101 so; 24 M, up to 30,000, 710 and 124.  512 sums: 20 M even entries 193 us with
+// 512 or 1,024, 32 lanes 202 and 218.
+// Seven CTAs an SM fit in 72 registers a thread: 8 M entries of 300 values, 2.2 waves of six CTAs
+// 115 us, 1.9 of seven 91; eight spill, 94.
+// Packets are shared by 4 warps where they fill the chip that deep, and by as many as it takes
+// (up to 32) where there are few of them, in shorter segments then: 204 packets 110 us with 4
+// warps, 59 with the CTA decoder, 46 so; 12 packets 59, 30 and 17.
+constexpr int DIVS_CTAS = 7;
+constexpr int DIVS_SUMS = 512;
 
-__host__ __device__ __forceinline__ int div_segment_entries(int L)
+int div_warps_per_packet(int64_t packets, int num_sms)
 {
+	const int64_t w = (int64_t) num_sms * DIVS_CTAS * 4 / (packets > 0 ? packets : 1);
+	return w >= 32 ? 32 : w >= 16 ? 16 : w >= 8 ? 8 : 4;
+}
+
+int div_segment_entries(int L, int warps)
+{
+	if (warps > 8)
+		return L <= 8 ? 64 : 8 * L;
 	return L <= 16 ? 256 : 16 * L;
 }
 
@@ -1092,10 +1112,16 @@ __device__ __forceinline__ void prefetch_l1(const uint8_t * p, const uint8_t * e
 		asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
 }
 
-template <int L>
-__global__ void __launch_bounds__(DIVS_THREADS, 6) div_segment_kernel(DivSegArgs a)
+// Sums a row in a packet of nrows <= DEC_MAX_ROWS rows: a power of two, nrows of them in DIVS_SUMS.
+__device__ __forceinline__ uint32_t div_copies(int64_t nrows)
 {
-	__shared__ double ys[DEC_MAX_ROWS];
+	return 1u << min(5, 31 - __clz(max(DIVS_SUMS / max((int) nrows, 1), 1)));
+}
+
+template <int L, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, WARPS > 4 ? 32 / WARPS : DIVS_CTAS) div_segment_kernel(DivSegArgs a)
+{
+	__shared__ double ys[DIVS_SUMS];
 	release_next();
 	const int64_t p = blockIdx.x;
 	const int t = threadIdx.x & 31, l = t & (L - 1);
@@ -1104,12 +1130,13 @@ __global__ void __launch_bounds__(DIVS_THREADS, 6) div_segment_kernel(DivSegArgs
 	const int64_t row_min = ld_u32(h + 12), col_min = ld_u32(h + 16);
 	const int row_bits = h[20], col_bits = h[21];
 	const int64_t nrf = ld_u32(h + 24);
-	const Coords coords(h + 28 + 4 * L + 8 * nrf, row_bits, col_bits);
+	Coords coords(h + 28 + 4 * L + 8 * nrf, row_bits, col_bits);
+	// kept in registers, not worked out again for each entry (4 lanes, 20 M values: 211 us, 193 so)
+	asm volatile("" : "+r"(coords.cb), "+r"(coords.row_bits), "+r"(coords.mask), "+r"(coords.rmask), "+r"(coords.cmask));
 	const uint8_t * codes = coords.base + coords.cb * nv;
 	const uint8_t * lanes = codes + nu;
 	const double * __restrict__ x = a.x + col_min;
 	const int s_end = a.pkt_seg[p + 1];
-	constexpr int WARPS = DIVS_THREADS / 32;
 	int s = a.pkt_seg[p] + (threadIdx.x >> 5);
 	// a segment's descriptor and places, and its lines asked of L1: the warp runs one ahead
 	int4 A, B;
@@ -1136,7 +1163,10 @@ __global__ void __launch_bounds__(DIVS_THREADS, 6) div_segment_kernel(DivSegArgs
 	};
 	fetch(s);
 	wait_previous();
-	for (int r = threadIdx.x; r < nrows && r < DEC_MAX_ROWS; r += blockDim.x)
+	// several sums a row, each of neighbouring threads
+	const uint32_t copies = div_copies(nrows), copy = t & (copies - 1);
+	auto add = [&](uint32_t row, double v) { atomicAdd(&ys[row * copies + copy], v); };
+	for (uint32_t r = threadIdx.x; r < nrows * copies && r < DIVS_SUMS; r += blockDim.x)
 		ys[r] = 0.0;
 	__syncthreads();
 	while (s < s_end) {
@@ -1173,7 +1203,7 @@ __global__ void __launch_bounds__(DIVS_THREADS, 6) div_segment_kernel(DivSegArgs
 				const uint64_t v = last + lane_inclusive_scan<L>(w.diff(code), t);
 				last = __shfl_sync(0xffffffffu, v, 32 - L + l);
 				if (u0 + t < nuniq)
-					atomicAdd(&ys[row], __longlong_as_double((long long) v) * xv);
+					add(row, __longlong_as_double((long long) v) * xv);
 				code = code1;
 				code1 = code2;
 				w = w1;
@@ -1212,7 +1242,7 @@ __global__ void __launch_bounds__(DIVS_THREADS, 6) div_segment_kernel(DivSegArgs
 				const int from = rest ? q : q * L + ((e - q * per) & (L - 1));
 				const double ve = __shfl_sync(0xffffffffu, vd, from & 31);
 				if (on)
-					atomicAdd(&ys[row], ve * xe);
+					add(row, ve * xe);
 			}
 		}
 	}
@@ -1220,13 +1250,35 @@ __global__ void __launch_bounds__(DIVS_THREADS, 6) div_segment_kernel(DivSegArgs
 	const int4 mt = a.meta[p];
 	for (int64_t r = (int64_t) mt.x + threadIdx.x; r < (int64_t) mt.y; r += blockDim.x) {
 		const int64_t rel = r - row_min;
-		if (rel < 0 || rel >= nrows) {
-			a.y[r] = 0.0;                                // empty rows between packets
-		} else if ((rel == 0 && (mt.z & 1)) || (rel == nrows - 1 && (mt.z & 2))) {
-			atomicAdd(&a.y[r], ys[rel]);                 // a row split across packets
-		} else {
-			a.y[r] = ys[rel];
-		}
+		const bool in = rel >= 0 && rel < nrows;
+		double sum = 0.0;                                    // stays 0 in empty rows between packets
+		for (uint32_t c = 0; c < copies && in; c++)
+			sum += ys[rel * copies + c];
+		if (in && ((rel == 0 && (mt.z & 1)) || (rel == nrows - 1 && (mt.z & 2))))
+			atomicAdd(&a.y[r], sum);                     // a row split across packets
+		else
+			a.y[r] = sum;
+	}
+}
+
+using DivSegFn = void (*)(DivSegArgs);
+
+template <int L>
+DivSegFn div_segment_fn(int warps)
+{
+	return warps == 32 ? div_segment_kernel<L, 32> : warps == 16 ? div_segment_kernel<L, 16>
+	     : warps == 8 ? div_segment_kernel<L, 8> : div_segment_kernel<L, 4>;
+}
+
+DivSegFn div_segment_fn(int L, int warps)
+{
+	switch (L) {
+	case 1: return div_segment_fn<1>(warps);
+	case 2: return div_segment_fn<2>(warps);
+	case 4: return div_segment_fn<4>(warps);
+	case 8: return div_segment_fn<8>(warps);
+	case 16: return div_segment_fn<16>(warps);
+	default: return div_segment_fn<32>(warps);
 	}
 }
 
@@ -1234,9 +1286,9 @@ __global__ void __launch_bounds__(DIVS_THREADS, 6) div_segment_kernel(DivSegArgs
 // or one by one in `parts` of their coordinates; then the incomplete position in parts.
 struct GroupSegments {
 	int64_t dv, md, np, parts, full, rest;
-	__device__ __forceinline__ GroupSegments(int64_t u, int64_t rf, int L)
+	__device__ __forceinline__ GroupSegments(int64_t u, int64_t rf, int L, int64_t S)
 	{
-		const int64_t S = div_segment_entries(L), step = 32 / L;
+		const int64_t step = 32 / L;
 		dv = u / L;
 		md = u % L;
 		parts = 1;
@@ -1252,13 +1304,13 @@ struct GroupSegments {
 	}
 };
 
-__global__ void div_seg_count_kernel(const int64_t * g_u, const int32_t * g_rf, int64_t G, int L, int64_t * count,
+__global__ void div_seg_count_kernel(const int64_t * g_u, const int32_t * g_rf, int64_t G, int L, int S, int64_t * count,
 		int64_t * nval)
 {
 	const int64_t g = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
 	if (g >= G)
 		return;
-	const GroupSegments k(g_u[g], g_rf[g], L);
+	const GroupSegments k(g_u[g], g_rf[g], L, S);
 	count[g] = k.full + k.rest;
 	nval[g] = (k.full > 0 ? k.full - k.parts : 0) + (k.dv > 0 ? k.rest : 0);     // segments that continue a lane
 }
@@ -1271,7 +1323,7 @@ __global__ void div_pkt_seg_kernel(const int32_t * pk_g0, const int64_t * seg_ba
 }
 
 // One thread per (segment, lane).
-__global__ void div_sync_kernel(const int64_t * seg_base, const int64_t * val_base, int64_t G, int64_t nseg, int L,
+__global__ void div_sync_kernel(const int64_t * seg_base, const int64_t * val_base, int64_t G, int64_t nseg, int L, int SE,
 		const int64_t * g_u, const int32_t * g_rf, const int64_t * g_ustart, const int64_t * g_start,
 		const int32_t * g_pkt, const int32_t * pk_g0, const int32_t * pk_j, const int64_t * gl_base, const int64_t * S,
 		const uint32_t * idx, const uint64_t * val_of, int4 * segs, uint32_t * seg_off, uint64_t * seg_val)
@@ -1289,8 +1341,8 @@ __global__ void div_sync_kernel(const int64_t * seg_base, const int64_t * val_ba
 		else
 			hi = mid - 1;
 	}
-	const int64_t g = lo, rf = g_rf[g], u = g_u[g], SE = div_segment_entries(L);
-	const GroupSegments k(u, rf, L);
+	const int64_t g = lo, rf = g_rf[g], u = g_u[g];
+	const GroupSegments k(u, rf, L, SE);
 	const int64_t j = sg - seg_base[g];
 	const bool rest = j >= k.full;
 	const int64_t pos = rest ? k.dv : j / k.parts * k.np;
@@ -1693,11 +1745,13 @@ int convert_div(Handle & h)
 	if (h.exec_kernel == 3) {
 		// segments of the decoder, each lane's place and value at their starts
 		DevBuf cnt3, nval3, base3, vbase3;
+		h.div_warps = div_warps_per_packet(NP, h.num_sms);
+		const int SE = div_segment_entries(L, h.div_warps);
 		SPMV_TRY(cnt3.alloc(G * 8, s));
 		SPMV_TRY(nval3.alloc(G * 8, s));
 		SPMV_TRY(base3.alloc((G + 1) * 8, s));
 		SPMV_TRY(vbase3.alloc((G + 1) * 8, s));
-		div_seg_count_kernel<<<(unsigned) ceil_div(G, 256), 256, 0, s>>>(g_u.as<int64_t>(), g_rf.as<int32_t>(), G, L,
+		div_seg_count_kernel<<<(unsigned) ceil_div(G, 256), 256, 0, s>>>(g_u.as<int64_t>(), g_rf.as<int32_t>(), G, L, SE,
 				cnt3.as<int64_t>(), nval3.as<int64_t>());
 		SPMV_CUDA_TRY(cudaGetLastError());
 		SPMV_TRY(scan_exclusive(cnt3.as<int64_t>(), base3.as<int64_t>(), G, s));
@@ -1714,7 +1768,7 @@ int convert_div(Handle & h)
 				h.d_pkt_seg);
 		SPMV_CUDA_TRY(cudaGetLastError());
 		div_sync_kernel<<<(unsigned) ceil_div(nseg * L, 256), 256, 0, s>>>(base3.as<int64_t>(), vbase3.as<int64_t>(), G, nseg,
-				L, g_u.as<int64_t>(), g_rf.as<int32_t>(), g_ustart.as<int64_t>(), g_start.as<int64_t>(),
+				L, SE, g_u.as<int64_t>(), g_rf.as<int32_t>(), g_ustart.as<int64_t>(), g_start.as<int64_t>(),
 				g_pkt.as<int32_t>(), pk_g0.as<int32_t>(), pk_j.as<int32_t>(), gl_base.as<int64_t>(), S.as<int64_t>(),
 				idx.as<uint32_t>(), val_of.as<uint64_t>(), h.d_segs, h.d_seg_off, h.d_seg_val);
 		SPMV_CUDA_TRY(cudaGetLastError());
@@ -1870,16 +1924,8 @@ int launch_div(Handle & h, const double * d_x, double * d_y, cudaStream_t s)
 		g.end = h.d_div + h.div_bytes;
 		g.x = d_x;
 		g.y = d_y;
-		void (*kern)(DivSegArgs) = nullptr;
-		switch (h.desc.vec_len) {
-		case 1: kern = div_segment_kernel<1>; break;
-		case 2: kern = div_segment_kernel<2>; break;
-		case 4: kern = div_segment_kernel<4>; break;
-		case 8: kern = div_segment_kernel<8>; break;
-		case 16: kern = div_segment_kernel<16>; break;
-		default: kern = div_segment_kernel<32>; break;
-		}
-		SPMV_CUDA_TRY(launch_overlapped(kern, (unsigned) h.num_packets, DIVS_THREADS, 0, s, g));
+		SPMV_CUDA_TRY(launch_overlapped(div_segment_fn(h.desc.vec_len, h.div_warps), (unsigned) h.num_packets,
+				(unsigned) h.div_warps * 32, 0, s, g));
 		return SPMV_OK;
 	}
 	DivArgs a;

@@ -160,6 +160,7 @@ struct Handle {
 	int4 * d_pkt_meta = nullptr;        // per packet: {y row start, y row end, flags, 0}
 	// segment decoder (exec_kernel 3): packets' segments, their descriptors, and each lane's
 	// payload byte and value at their starts
+	int div_warps = 0;                  // warps a packet
 	int32_t * d_pkt_seg = nullptr;
 	int4 * d_segs = nullptr;
 	uint32_t * d_seg_off = nullptr;

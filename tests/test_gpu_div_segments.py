@@ -44,3 +44,21 @@ def test_segments_match_the_cta_decoder(sb, orc, kind, packet, L):
     gold, absy = orc.csr_gold(rp, ci, v, x)
     assert rel_row_error(y, gold, absy) <= TOL
     assert rel_row_error(y, y0, absy) <= TOL
+
+
+@pytest.mark.parametrize("packets", [100, 200, 400, 1500])
+@pytest.mark.parametrize("L", [4, 32])
+def test_long_rows_and_every_packet_width(sb, orc, L, packets):
+    """4 to 32 warps a packet by their number; packets of one long row and of many short ones."""
+    r = np.random.default_rng(packets + L)
+    n = 3000
+    lengths = r.integers(0, 5, packets * 16)
+    lengths[:packets // 100] = n                         # packets of one row: 32 sums a row
+    rp = np.zeros(len(lengths) + 1, np.int32)
+    np.cumsum(lengths, out=rp[1:])
+    ci = np.concatenate([np.sort(r.choice(n, k, replace=False)) for k in lengths]).astype(np.int32)
+    m, nnz = len(lengths), int(rp[-1])
+    v, x = _values("mixed", nnz, r), r.uniform(-1, 1, n)
+    y = sb.csr_to_format(rp, ci, v, m, n, nnz, format="div_rf", vec_len=L, div_packet_vals=64).spmv(x, np.full(m, 1.0))
+    gold, absy = orc.csr_gold(rp, ci, v, x)
+    assert rel_row_error(y, gold, absy) <= TOL
