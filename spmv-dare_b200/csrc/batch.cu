@@ -7,7 +7,7 @@
 //   row tiles       the default of mixed batches: one layout (tile_kernels.cu) over the rows of
 //                   all matrices, each slice with its format's arithmetic, ranges of equal cost
 //                   dealt over the whole batch.  48 matrices of 1,000 to 100,000 rows (34 M
-//                   entries, the four formats in turn): 114 us against 486 for the work queue,
+//                   entries, the four formats in turn): 98 us against 486 for the work queue,
 //                   whose CTAs wait at two barriers a block and give a long row to one thread;
 //   work queue      a given block size, stage count or CTA size, tolerance mode, slices of 1 or
 //                   2 rows, or where the layout does not pay: the matrices' staged-block tables

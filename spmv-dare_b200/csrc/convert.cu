@@ -480,7 +480,7 @@ static int build_tiled_cols(Handle & h, const int32_t * d_P, int64_t U, int V)
 // 57 8.0 and 9.6; from 7.6 M entries on row tiles are the faster (csr_naive 25.9 and 25.1 us
 // there, 50.4 and 37.0 with 10.7 M; sell_sorted 23.9 and 19.3 with 4.1 M).  The FP32
 // variant: 14.7 and 18.9 us with 2.6 M entries, 24.0 and 23.2 with 4.7 M, 108 and 68 with 24 M
-// scattered ones, 170 both on the 4M-row matrix.  SELL-C-sigma gains at every size: its other
+// scattered ones, 167 and 161 on the 4M-row matrix.  SELL-C-sigma gains at every size: its other
 // kernels give a slice to a warp or two (1,671 rows 18.9 and 3.6 us).
 constexpr int64_t TILE_ENTRIES = 3500000;
 
@@ -540,9 +540,9 @@ int build_row_tiles(Handle & h)
 			[&h](void ** p, size_t bytes) { return h.alloc((uint8_t **) p, (int64_t) bytes); });
 }
 
-// Kernel choice: -1 = the format's default (the register-tiled warp kernel for slices of 32
-// rows, the tiled warp-specialised kernel for wider SELL-C-sigma slices, the warp-specialised
-// kernel otherwise: the fastest of each on the 4M-row configuration); 0 = CTA
+// Kernel choice: -1 = the format's default (row tiles where tiles_default says so; else the
+// register-tiled warp kernel for slices of 32 rows, the tiled warp-specialised kernel for wider
+// SELL-C-sigma slices, the warp-specialised kernel otherwise); 0 = CTA
 // staged kernel; 1 = direct column-major kernel (slices of >= 32 rows only); 2 =
 // warp-autonomous staged kernel (slices of <= 32 rows); 3 = CTA staged kernel with the next
 // block's gather overlapping this block's rows; 4 = warp-specialised staged kernel; 5 = CTA
@@ -565,7 +565,7 @@ int build_exec(Handle & h, const int32_t * d_P, int64_t U, int V)
 		}
 	}
 	if (k < 0) {
-		// measured on the 4M-row matrix: kernel 4 is the fastest for csr_naive (0.193 ms),
+		// of these, measured on the 4M-row matrix: kernel 4 is the fastest for csr_naive (0.193 ms),
 		// csr_vec, and sell / sell_sorted with slices of up to 16 rows; kernel 10 for slices of
 		// exactly 32 rows (SELL-C-sigma 0.213 ms against kernel 8's 0.255-0.266, sell 0.197,
 		// sell_sorted 0.217); kernel 8 for SELL-C-sigma with wider slices.  A requested staging

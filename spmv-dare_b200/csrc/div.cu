@@ -1521,8 +1521,9 @@ int convert_div(Handle & h)
 		set_error(SPMV_ERR_ARG, "DIV-RF: vec_len %d above %d", L, DEC_THREADS);
 		return SPMV_ERR_ARG;
 	}
-	// decoder: 2 = one warp per packet, one lane per lane stream (32 lanes only; the default
-	// there); 0 = one CTA per packet, lanes shared by several threads (any lane count)
+	// decoder: 2 = one warp per packet, one lane per lane stream (32 lanes only, taken there when
+	// stages, block_nnz or ctas_per_sm are given); 0 = one CTA per packet, lanes shared by several
+	// threads (any lane count)
 	h.exec_kernel = h.desc.kernel < 0 ? (L == 32 ? 2 : 0) : h.desc.kernel;
 	if (h.exec_kernel != 0 && !(h.exec_kernel == 2 && L == 32)) {
 		set_error(SPMV_ERR_ARG, "DIV-RF: kernel %d unavailable (0, or 2 with vec_len 32)", h.desc.kernel);

@@ -23,9 +23,9 @@
 // alone, DRAM (csr_naive on 4M rows 174 us, 6.0 TB/s).  Measured in a loop over three matrices,
 // before (warp-specialised CTAs staging blocks in shared memory, where row threads met in banks;
 // SELL-C-sigma: a queue of register tiles with 16 warps an SM) and now: csr_naive 4M rows
-// 213 -> 198 us, SELL-C-sigma 4M rows 224 -> 207, csr_vec 1M rows 150 -> 95, SELL 2M rows
-// 160 -> 144, sell_sorted 700k rows 101 -> 64.  Tried: x transposed between lanes by shuffles
-// (16 warps of 114 registers an SM: 255 us on csr_naive), CTAs of 256 threads (202) and 128
+// 213 -> 191 us, SELL-C-sigma 4M rows 224 -> 202, csr_vec 1M rows 150 -> 93, SELL 2M rows
+// 160 -> 132, sell_sorted 700k rows 101 -> 62.  Tried on csr_naive when it took 198: x transposed between
+// lanes by shuffles (16 warps of 114 registers an SM: 255 us), CTAs of 256 threads (202) and 128
 // (199), bulk prefetches into L2 (1-10% slower), columns and x one tile further ahead (209),
 // four threads a row straight from CSR (csr_vec 143: a wavefront per row and request).
 //
