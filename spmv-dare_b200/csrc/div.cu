@@ -999,22 +999,41 @@ __global__ void __launch_bounds__(DIVW_WARPS * 32, MINB) div_warp_kernel(DivArgs
 // 512 or 1,024, 32 lanes 202 and 218.
 // Seven CTAs an SM fit in 72 registers a thread: 8 M entries of 300 values, 2.2 waves of six CTAs
 // 115 us, 1.9 of seven 91; eight spill, 94.
-// Packets are shared by 4 warps where they fill the chip that deep, and by as many as it takes
-// (up to 32) where there are few of them, in shorter segments then: 204 packets 110 us with 4
-// warps, 59 with the CTA decoder, 46 so; 12 packets 59, 30 and 17.
+// Warps a packet (4, 8, 16 or 32, in shorter segments from 8 on): from the waves of mean packets and
+// the largest packet, a warp's share of the larger; twice the warps only where that nearly
+// halves, since 64 registers a thread spill (371 packets 30 us with 16 warps, in two waves).  204 packets 110 us with 4 warps, 59 with the CTA
+// decoder, 46 so; 12 packets 59, 30 and 17; 571 packets 43, 43 and 30 with 8 warps; 782 44 with 4
+// and 46 with 8; 1,000 packets, some of long rows and four times the mean, 119, 121 and 74 with 8.
 constexpr int DIVS_CTAS = 7;
 constexpr int DIVS_SUMS = 512;
 
-int div_warps_per_packet(int64_t packets, int num_sms)
+int div_warps_per_packet(int64_t packets, int64_t entries, int64_t largest, int num_sms)
 {
-	const int64_t w = (int64_t) num_sms * DIVS_CTAS * 4 / (packets > 0 ? packets : 1);
-	return w >= 32 ? 32 : w >= 16 ? 16 : w >= 8 ? 8 : 4;
+	auto time = [&](int w) {
+		const int64_t at_once = (int64_t) num_sms * (w > 4 ? 32 / w : DIVS_CTAS);
+		const double waves = (double) entries / (packets < at_once ? packets : at_once);
+		return (waves > largest ? waves : (double) largest) / w;
+	};
+	int w = 4;
+	while (packets > 0 && w < 32 && time(2 * w) * 1.9 <= time(w))
+		w *= 2;
+	return w;
+}
+
+__global__ void div_largest_kernel(const int32_t * pk_nv, int64_t NP, int32_t * largest)
+{
+	const int64_t p = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
+	const int v = __reduce_max_sync(0xffffffffu, p < NP ? pk_nv[p] : 0);
+	if ((threadIdx.x & 31) == 0)
+		atomicMax(largest, v);
 }
 
 int div_segment_entries(int L, int warps)
 {
 	if (warps > 8)
 		return L <= 8 ? 64 : 8 * L;
+	if (warps == 8)
+		return L <= 8 ? 128 : 8 * L;
 	return L <= 16 ? 256 : 16 * L;
 }
 
@@ -1118,8 +1137,8 @@ __device__ __forceinline__ uint32_t div_copies(int64_t nrows)
 	return 1u << min(5, 31 - __clz(max(DIVS_SUMS / max((int) nrows, 1), 1)));
 }
 
-template <int L, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32, WARPS > 4 ? 32 / WARPS : DIVS_CTAS) div_segment_kernel(DivSegArgs a)
+template <int L, int WARPS, int CTAS = (WARPS > 4 ? 32 / WARPS : DIVS_CTAS)>
+__global__ void __launch_bounds__(WARPS * 32, CTAS) div_segment_kernel(DivSegArgs a)
 {
 	__shared__ double ys[DIVS_SUMS];
 	release_next();
@@ -1263,22 +1282,24 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS > 4 ? 32 / WARPS : DIVS_CTAS
 
 using DivSegFn = void (*)(DivSegArgs);
 
+// 8 warps, three CTAs an SM and no spills, where that is all the packets need: 430 packets 29 us with
+// four, 23 so, 27 with the CTA decoder.
 template <int L>
-DivSegFn div_segment_fn(int warps)
+DivSegFn div_segment_fn(int warps, bool three)
 {
 	return warps == 32 ? div_segment_kernel<L, 32> : warps == 16 ? div_segment_kernel<L, 16>
-	     : warps == 8 ? div_segment_kernel<L, 8> : div_segment_kernel<L, 4>;
+	     : warps == 8 ? (three ? div_segment_kernel<L, 8, 3> : div_segment_kernel<L, 8>) : div_segment_kernel<L, 4>;
 }
 
-DivSegFn div_segment_fn(int L, int warps)
+DivSegFn div_segment_fn(int L, int warps, bool three)
 {
 	switch (L) {
-	case 1: return div_segment_fn<1>(warps);
-	case 2: return div_segment_fn<2>(warps);
-	case 4: return div_segment_fn<4>(warps);
-	case 8: return div_segment_fn<8>(warps);
-	case 16: return div_segment_fn<16>(warps);
-	default: return div_segment_fn<32>(warps);
+	case 1: return div_segment_fn<1>(warps, three);
+	case 2: return div_segment_fn<2>(warps, three);
+	case 4: return div_segment_fn<4>(warps, three);
+	case 8: return div_segment_fn<8>(warps, three);
+	case 16: return div_segment_fn<16>(warps, three);
+	default: return div_segment_fn<32>(warps, three);
 	}
 }
 
@@ -1746,7 +1767,15 @@ int convert_div(Handle & h)
 	if (h.exec_kernel == 3) {
 		// segments of the decoder, each lane's place and value at their starts
 		DevBuf cnt3, nval3, base3, vbase3;
-		h.div_warps = div_warps_per_packet(NP, h.num_sms);
+		DevBuf most;
+		int32_t largest = 0;
+		SPMV_TRY(most.alloc(4, s));
+		SPMV_CUDA_TRY(cudaMemsetAsync(most.p, 0, 4, s));
+		div_largest_kernel<<<(unsigned) ceil_div(NP, 256), 256, 0, s>>>(pk_nv.as<int32_t>(), NP, most.as<int32_t>());
+		SPMV_CUDA_TRY(cudaGetLastError());
+		SPMV_CUDA_TRY(cudaMemcpyAsync(&largest, most.p, 4, cudaMemcpyDeviceToHost, s));
+		SPMV_CUDA_TRY(cudaStreamSynchronize(s));
+		h.div_warps = div_warps_per_packet(NP, nnz, largest, h.num_sms);
 		const int SE = div_segment_entries(L, h.div_warps);
 		SPMV_TRY(cnt3.alloc(G * 8, s));
 		SPMV_TRY(nval3.alloc(G * 8, s));
@@ -1925,7 +1954,8 @@ int launch_div(Handle & h, const double * d_x, double * d_y, cudaStream_t s)
 		g.end = h.d_div + h.div_bytes;
 		g.x = d_x;
 		g.y = d_y;
-		SPMV_CUDA_TRY(launch_overlapped(div_segment_fn(h.desc.vec_len, h.div_warps), (unsigned) h.num_packets,
+		SPMV_CUDA_TRY(launch_overlapped(div_segment_fn(h.desc.vec_len, h.div_warps,
+				h.num_packets <= 3 * h.num_sms), (unsigned) h.num_packets,
 				(unsigned) h.div_warps * 32, 0, s, g));
 		return SPMV_OK;
 	}
