@@ -247,7 +247,7 @@ int build_batch_tiles(spmv_batch * b, int32_t count, const int32_t * const * row
 		int sms = 0;
 		cudaGetDevice(&b->device);
 		cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
-		st = spmv::build_tiles(b->tiles, src, false, true, sms, b->stream, [b](void ** p, size_t bytes) {
+		st = spmv::build_tiles(b->tiles, src, 0, false, true, sms, b->stream, [b](void ** p, size_t bytes) {
 			return balloc(b, (uint8_t **) p, (int64_t) bytes);
 		});
 	}
@@ -271,7 +271,7 @@ int enqueue(spmv_batch * b, const double * d_x, double * d_y, cudaStream_t s)
 	if (b->merged)
 		return spmv_run_device(b->merged, d_x, d_y, s);
 	if (b->tiles.built)
-		return spmv::launch_tiles(b->tiles, SPMV_FMT_SELL, 1, d_x, d_y, s);
+		return spmv::launch_tiles(b->tiles, d_x, d_y, s);
 	SPMV_CUDA_TRY(cudaMemsetAsync(b->d_counter, 0, sizeof(unsigned long long), s));
 	if (b->nblocks == 0)
 		return SPMV_OK;

@@ -536,7 +536,9 @@ TileSource tile_source(const Handle & h)
 
 int build_row_tiles(Handle & h)
 {
-	return build_tiles(h.tiles, {tile_source(h)}, h.desc.values == SPMV_VALUES_F32, false, h.num_sms, h.stream,
+	const bool f32 = h.desc.values == SPMV_VALUES_F32;
+	const int lanes = h.desc.format == SPMV_FMT_CSR_VEC && !f32 ? h.desc.vec_len : 0;
+	return build_tiles(h.tiles, {tile_source(h)}, lanes, f32, false, h.num_sms, h.stream,
 			[&h](void ** p, size_t bytes) { return h.alloc((uint8_t **) p, (int64_t) bytes); });
 }
 

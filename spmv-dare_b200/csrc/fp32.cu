@@ -1317,7 +1317,7 @@ int launch_spmv_f32(Handle & h, const float * d_x, float * d_y, cudaStream_t s)
 	if (h.desc.format == SPMV_FMT_SELL_C_S)
 		return launch_sliced_f32(h, d_x, d_y, s);
 	if (h.exec_kernel == 11)
-		return launch_tiles(h.tiles, h.desc.format, 1, d_x, d_y, s);
+		return launch_tiles(h.tiles, d_x, d_y, s);
 	if (h.exec_kernel == 7) {
 		if (h.num_empty_rows > 0) {
 			zero_rows_f32_kernel<<<(unsigned) ceil_div(h.num_empty_rows, 256), 256, 0, s>>>(h.d_empty_rows,

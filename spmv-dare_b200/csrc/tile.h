@@ -47,6 +47,8 @@ struct TilePlan {
 	bool built = false;
 	int32_t pad_col = PAD_OWN;
 	bool f32 = false, mixed = false, wide = false, staged = false;
+	bool split = false;          // csr_naive arithmetic (MIXED batches: by slice)
+	int lanes = 0;               // csr_vec: its lanes; 0: rows summed in order
 	int32_t * sptr = nullptr;
 	int32_t * tcols = nullptr;
 	void * vals = nullptr;
@@ -59,9 +61,9 @@ struct TilePlan {
 };
 
 // Builds the layout; p.built stays false where it does not pay (padding above a third of the
-// entries) or does not fit 32-bit indices.
-int build_tiles(TilePlan & p, const std::vector<TileSource> & src, bool f32, bool mixed, int num_sms, cudaStream_t s,
-		const std::function<int(void **, size_t)> & alloc);
-int launch_tiles(const TilePlan & p, int format, int lanes, const void * x, void * y, cudaStream_t s);
+// entries) or does not fit 32-bit indices.  lanes: 4 or 8 for csr_vec's row sums, else 0.
+int build_tiles(TilePlan & p, const std::vector<TileSource> & src, int lanes, bool f32, bool mixed, int num_sms,
+		cudaStream_t s, const std::function<int(void **, size_t)> & alloc);
+int launch_tiles(const TilePlan & p, const void * x, void * y, cudaStream_t s);
 
 }  // namespace spmv

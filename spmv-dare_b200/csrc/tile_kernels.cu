@@ -863,7 +863,8 @@ using TileFn = void (*)(TileArgs);
 // buffer.  Rows that share columns decide: 1.5M rows of 40, no neighbours, pairs of equal rows
 // 170 us copied and 154 staged (0.29 lines an entry saved), a third in such pairs 177 and 174
 // (0.13), none 192 and 199; csr_naive on 4M rows (0.06) 196 and 206; SELL 2M rows (0.17) 140 and
-// 134.  Measured on a sample of the slices at conversion.
+// 134.  Measured on a sample of the slices at conversion, for the sums in order of a single
+// FP64 matrix: csr_vec's lanes, FP32 and mixed batches have no such build.
 //
 // Two builds of the plain sums.  WIDE (12 CTAs an SM, 80 registers a thread, a tile's values
 // loaded after the tile before it is summed) for matrices of many ranges a warp: csr_naive on
@@ -871,28 +872,33 @@ using TileFn = void (*)(TileArgs);
 // a lone slice against 0.40, csr_naive on 60,000 equal rows of 19 5.25 us against 5.65.
 constexpr int WIDE_CTAS = 12, DEEP_CTAS = 10, LANES_CTAS = 9;
 
-TileFn tile_fn(int format, int lanes, bool f32, bool mixed, bool wide, bool staged)
+// The arithmetic first, its builds after: a build stands for one order of operations.
+TileFn tile_fn(const TilePlan & p)
 {
-	if (mixed)
-		return wide ? tile_kernel<Sum::MIXED, WIDE_CTAS, false> : tile_kernel<Sum::MIXED, DEEP_CTAS, true>;
-	if (f32)
-		return wide ? tile_kernel<Sum::DOT2, WIDE_CTAS, false> : tile_kernel<Sum::DOT2, DEEP_CTAS, true>;
-	if (wide && staged)
-		return format == SPMV_FMT_CSR_NAIVE ? tile_kernel<Sum::NAIVE, WIDE_CTAS, false, true>
-		                                    : tile_kernel<Sum::FMA, WIDE_CTAS, false, true>;
-	if (format == SPMV_FMT_CSR_NAIVE)
-		return wide ? tile_kernel<Sum::NAIVE, WIDE_CTAS, false> : tile_kernel<Sum::NAIVE, DEEP_CTAS, true>;
-	if (format == SPMV_FMT_CSR_VEC)
-		return lanes == 8 ? tile_kernel<Sum::LANES8, LANES_CTAS, false> : tile_kernel<Sum::LANES4, LANES_CTAS, false>;
-	return wide ? tile_kernel<Sum::FMA, WIDE_CTAS, false> : tile_kernel<Sum::FMA, DEEP_CTAS, true>;
+	if (p.mixed)
+		return p.wide ? tile_kernel<Sum::MIXED, WIDE_CTAS, false> : tile_kernel<Sum::MIXED, DEEP_CTAS, true>;
+	if (p.f32)
+		return p.wide ? tile_kernel<Sum::DOT2, WIDE_CTAS, false> : tile_kernel<Sum::DOT2, DEEP_CTAS, true>;
+	if (p.lanes)
+		return p.lanes == 8 ? tile_kernel<Sum::LANES8, LANES_CTAS, false> : tile_kernel<Sum::LANES4, LANES_CTAS, false>;
+	if (p.split)
+		return p.staged ? tile_kernel<Sum::NAIVE, WIDE_CTAS, false, true>
+		     : p.wide   ? tile_kernel<Sum::NAIVE, WIDE_CTAS, false>
+		                : tile_kernel<Sum::NAIVE, DEEP_CTAS, true>;
+	return p.staged ? tile_kernel<Sum::FMA, WIDE_CTAS, false, true>
+	     : p.wide   ? tile_kernel<Sum::FMA, WIDE_CTAS, false>
+	                : tile_kernel<Sum::FMA, DEEP_CTAS, true>;
 }
 
 }  // namespace
 
-int build_tiles(TilePlan & p, const std::vector<TileSource> & src, bool f32, bool mixed, int num_sms, cudaStream_t s,
-		const std::function<int(void **, size_t)> & alloc)
+int build_tiles(TilePlan & p, const std::vector<TileSource> & src, int lanes, bool f32, bool mixed, int num_sms,
+		cudaStream_t s, const std::function<int(void **, size_t)> & alloc)
 {
 	p.built = false;
+	p.f32 = f32;
+	p.mixed = mixed;
+	p.lanes = lanes;
 	int64_t nslots = 0, entries = 0, rows = 0;
 	std::vector<int64_t> slot0;
 	for (const TileSource & t : src) {
@@ -1004,7 +1010,7 @@ int build_tiles(TilePlan & p, const std::vector<TileSource> & src, bool f32, boo
 	p.nranges = ceil_div(cost, share);
 	p.wide = cost > 4 * warps * RANGE_COST;
 	p.staged = false;
-	if (p.wide && !f32) {
+	if (p.wide && !f32 && !mixed && lanes == 0) {
 		DevBuf lines;
 		unsigned long long l[2];
 		SPMV_TRY(lines.alloc(sizeof(l), s));
@@ -1022,14 +1028,13 @@ int build_tiles(TilePlan & p, const std::vector<TileSource> & src, bool f32, boo
 	p.grid = ceil_div(p.nranges + nlong, TILE_WARPS);
 	if (p.grid < nlong)
 		p.grid = nlong;
-	p.f32 = f32;
-	p.mixed = mixed;
+	p.split = src[0].split;
 	p.pad_col = src[0].pad_col;
 	p.built = true;
 	return SPMV_OK;
 }
 
-int launch_tiles(const TilePlan & p, int format, int lanes, const void * x, void * y, cudaStream_t s)
+int launch_tiles(const TilePlan & p, const void * x, void * y, cudaStream_t s)
 {
 	if (p.grid == 0)
 		return SPMV_OK;
@@ -1047,8 +1052,7 @@ int launch_tiles(const TilePlan & p, int format, int lanes, const void * x, void
 	a.nranges = (int) p.nranges;
 	a.longs = p.longs;
 	a.nlong = (int) p.nlong;
-	SPMV_CUDA_TRY(launch_overlapped(tile_fn(format, lanes, p.f32, p.mixed, p.wide, p.staged), (unsigned) p.grid, TILE_THREADS, 0,
-			s, a));
+	SPMV_CUDA_TRY(launch_overlapped(tile_fn(p), (unsigned) p.grid, TILE_THREADS, 0, s, a));
 	return SPMV_OK;
 }
 
