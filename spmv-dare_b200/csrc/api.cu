@@ -41,6 +41,7 @@ cudaError_t pool_alloc(void ** p, size_t bytes, Pool kind, cudaStream_t s)
 	constexpr int MOST = 64;
 	static std::mutex lock;
 	static cudaMemPool_t pools[MOST][2];
+	static void * word[MOST];
 	int dev = 0;
 	cudaError_t e = cudaGetDevice(&dev);
 	if (e != cudaSuccess || dev >= MOST)
@@ -48,6 +49,9 @@ cudaError_t pool_alloc(void ** p, size_t bytes, Pool kind, cudaStream_t s)
 	cudaMemPool_t both[2];
 	{
 		std::lock_guard<std::mutex> hold(lock);
+		// a word that stays, so that the last handle's error word does not take its 2 MB of mapped memory along
+		if (!word[dev] && (e = cudaMalloc(&word[dev], sizeof(int))) != cudaSuccess)
+			return e;
 		for (int k = 0; k < 2; k++) {
 			if (!pools[dev][k]) {
 				cudaMemPoolProps props{};
@@ -185,14 +189,22 @@ static void release_handle(Handle & h)
 {
 	if (!h.stream)
 		return;                    // no device yet, so nothing allocated
-	// the caller's SpMVs may run on any stream: the memory goes back once all work is done
 	int cur = h.device;
 	cudaGetDevice(&cur);
 	if (cur != h.device)
 		cudaSetDevice(h.device);
-	cudaDeviceSynchronize();
+	// The caller's SpMVs may run on any stream, and the pools hand memory on at once: it goes back
+	// once all work is done.  cudaFree waits for that (every handle has a plain allocation, its
+	// error word), also while a stream is captured, where cudaDeviceSynchronize is refused and
+	// ends the capture.  Where cudaFree is refused, the pools do not get the memory back.
+	const BesideCapture beside;
+	bool idle = true;
 	for (const Handle::Allocation & a : h.allocations)
-		a.pooled ? cudaFreeAsync(a.p, h.stream) : cudaFree(a.p);
+		if (!a.pooled)
+			idle = cudaFree(a.p) == cudaSuccess && idle;
+	for (const Handle::Allocation & a : h.allocations)
+		if (a.pooled && idle)
+			cudaFreeAsync(a.p, h.stream);
 	h.allocations.clear();
 	cudaStreamDestroy(h.stream);
 	h.stream = nullptr;
@@ -238,7 +250,7 @@ static int init_device(Handle & h)
 	SPMV_CUDA_TRY(cudaGetDevice(&h.device));
 	SPMV_CUDA_TRY(cudaDeviceGetAttribute(&h.num_sms, cudaDevAttrMultiProcessorCount, h.device));
 	SPMV_CUDA_TRY(cudaStreamCreateWithFlags(&h.stream, cudaStreamNonBlocking));
-	SPMV_TRY(h.alloc(&h.d_err, 1));
+	SPMV_TRY(h.alloc(&h.d_err, 1, false));
 	SPMV_CUDA_TRY(cudaMemsetAsync(h.d_err, 0, sizeof(int), h.stream));
 	return SPMV_OK;
 }

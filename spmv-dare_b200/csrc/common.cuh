@@ -46,6 +46,14 @@ constexpr size_t POOL_MOST_BYTES = (size_t) 128 << 20;
 enum class Pool { SCRATCH, HANDLE };
 cudaError_t pool_alloc(void ** p, size_t bytes, Pool pool, cudaStream_t s);
 
+// While it lives, memory calls of this thread go through beside a stream capture, its own or
+// another thread's, which they otherwise end.
+struct BesideCapture {
+	cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+	BesideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+	~BesideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // Device-side error word (one per handle): first error wins.
 #define DEV_ERR_TIMEOUT 1
 #define DEV_ERR_BOUNDS  2

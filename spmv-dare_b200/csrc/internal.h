@@ -201,11 +201,11 @@ struct Handle {
 	std::string name;
 
 	template <typename T>
-	int alloc(T ** p, int64_t count)
+	int alloc(T ** p, int64_t count, bool may_pool = true)
 	{
 		size_t bytes = (size_t) (count > 0 ? count : 1) * sizeof(T);
 		const auto t0 = std::chrono::steady_clock::now();
-		const bool pooled = bytes <= POOL_MOST_BYTES;
+		const bool pooled = may_pool && bytes <= POOL_MOST_BYTES;
 		cudaError_t e = pooled ? pool_alloc((void **) p, bytes, Pool::HANDLE, stream) : cudaMalloc((void **) p, bytes);
 		alloc_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
 		if (e != cudaSuccess) {
