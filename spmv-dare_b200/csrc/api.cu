@@ -2,6 +2,7 @@
 #include <stdarg.h>
 #include <string.h>
 
+#include <atomic>
 #include <chrono>
 #include <mutex>
 #include <string>
@@ -36,52 +37,72 @@ void clear_error()
 }
 
 // Pools are made on first use and kept for the process.
-cudaError_t pool_alloc(void ** p, size_t bytes, Pool kind, cudaStream_t s)
+struct DevicePools {
+	cudaMemPool_t pool[2] = {};
+	void * word = nullptr;                 // stays, so that the last handle's error word does not unmap its 2 MB
+	std::atomic<int64_t> live{0};          // bytes of handles in the HANDLE pool
+};
+
+static cudaError_t device_pools(DevicePools ** out)
 {
 	constexpr int MOST = 64;
 	static std::mutex lock;
-	static cudaMemPool_t pools[MOST][2];
-	static void * word[MOST];
+	static DevicePools all[MOST];
 	int dev = 0;
 	cudaError_t e = cudaGetDevice(&dev);
 	if (e != cudaSuccess || dev >= MOST)
 		return e != cudaSuccess ? e : cudaErrorInvalidDevice;
-	cudaMemPool_t both[2];
-	{
-		std::lock_guard<std::mutex> hold(lock);
-		// a word that stays, so that the last handle's error word does not take its 2 MB of mapped memory along
-		if (!word[dev] && (e = cudaMalloc(&word[dev], sizeof(int))) != cudaSuccess)
+	DevicePools & d = all[dev];
+	std::lock_guard<std::mutex> hold(lock);
+	if (!d.word && (e = cudaMalloc(&d.word, sizeof(int))) != cudaSuccess)
+		return e;
+	for (cudaMemPool_t & q : d.pool) {
+		if (q)
+			continue;
+		cudaMemPoolProps props{};
+		props.allocType = cudaMemAllocationTypePinned;
+		props.location.type = cudaMemLocationTypeDevice;
+		props.location.id = dev;
+		unsigned long long keep = POOL_KEEP_BYTES;
+		int look = 0;          // at other streams' progress: every allocation would, 2.8 us a stream that is alive
+		cudaMemPool_t made = nullptr;
+		if ((e = cudaMemPoolCreate(&made, &props)) != cudaSuccess)
 			return e;
-		for (int k = 0; k < 2; k++) {
-			if (!pools[dev][k]) {
-				cudaMemPoolProps props{};
-				props.allocType = cudaMemAllocationTypePinned;
-				props.location.type = cudaMemLocationTypeDevice;
-				props.location.id = dev;
-				unsigned long long keep = POOL_KEEP_BYTES;
-				int look = 0;          // at other streams' progress: every allocation would, 2.8 us a stream that is alive
-				cudaMemPool_t made = nullptr;
-				if ((e = cudaMemPoolCreate(&made, &props)) != cudaSuccess)
-					return e;
-				if ((e = cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess ||
-						(e = cudaMemPoolSetAttribute(made, cudaMemPoolReuseAllowOpportunistic, &look)) != cudaSuccess) {
-					cudaMemPoolDestroy(made);
-					return e;
-				}
-				pools[dev][k] = made;
-			}
-			both[k] = pools[dev][k];
+		if ((e = cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess ||
+				(e = cudaMemPoolSetAttribute(made, cudaMemPoolReuseAllowOpportunistic, &look)) != cudaSuccess) {
+			cudaMemPoolDestroy(made);
+			return e;
 		}
+		q = made;
 	}
-	e = cudaMallocFromPoolAsync(p, bytes, both[(int) kind], s);
+	*out = &d;
+	return cudaSuccess;
+}
+
+cudaError_t pool_alloc(void ** p, size_t bytes, Pool kind, cudaStream_t s)
+{
+	DevicePools * d = nullptr;
+	cudaError_t e = device_pools(&d);
+	if (e != cudaSuccess)
+		return e;
+	e = cudaMallocFromPoolAsync(p, bytes, d->pool[(int) kind], s);
 	if (e == cudaErrorMemoryAllocation) {
 		cudaGetLastError();
 		cudaDeviceSynchronize();
-		for (cudaMemPool_t q : both)
+		for (cudaMemPool_t q : d->pool)
 			cudaMemPoolTrimTo(q, 0);
-		e = cudaMallocFromPoolAsync(p, bytes, both[(int) kind], s);
+		e = cudaMallocFromPoolAsync(p, bytes, d->pool[(int) kind], s);
 	}
 	return e;
+}
+
+void pool_live(int64_t bytes)
+{
+	DevicePools * d = nullptr;
+	if (device_pools(&d) != cudaSuccess)
+		return;
+	unsigned long long keep = POOL_KEEP_BYTES + (unsigned long long) (d->live += bytes);
+	cudaMemPoolSetAttribute(d->pool[(int) Pool::HANDLE], cudaMemPoolAttrReleaseThreshold, &keep);
 }
 
 static const char * kNames[SPMV_NUM_FORMATS] = {
@@ -204,9 +225,11 @@ static void release_handle(Handle & h)
 	for (const Handle::Allocation & a : h.allocations)
 		if (!a.pooled)
 			idle = cudaFree(a.p) == cudaSuccess && idle;
+	int64_t live = 0;
 	for (const Handle::Allocation & a : h.allocations)
-		if (a.pooled && idle)
-			cudaFreeAsync(a.p, h.stream);
+		if (a.pooled && idle && cudaFreeAsync(a.p, h.stream) == cudaSuccess)
+			live += a.bytes;
+	pool_live(-live);
 	h.allocations.clear();
 	cudaStreamDestroy(h.stream);
 	h.stream = nullptr;

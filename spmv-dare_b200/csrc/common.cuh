@@ -36,9 +36,9 @@ int  last_status();
 // Stream-ordered allocations on the current device, from two pools per device of the library's
 // own: one for scratch, one for the arrays of handles up to POOL_MOST_BYTES each (larger ones are
 // plain allocations).  Mapping and unmapping memory cost a conversion more than its kernels, so
-// each pool keeps up to POOL_KEEP_BYTES of reserved memory between uses; an allocation that
+// each pool keeps up to POOL_KEEP_BYTES that nothing uses; an allocation that
 // fails gives all of it back first and tries again.  (One pool for both, or larger arrays in it,
-// put live arrays above that bound, and every synchronisation unmapped the scratch: 34 ms
+// put live arrays above the bound, and every synchronisation unmapped the scratch: 34 ms
 // against 12 for a 2M-row SELL conversion.)  A SELL-C-sigma conversion of 8.5 M host entries with
 // one SpMV: 12.8 ms with cudaMalloc and the default pool, 5.9 so.  The pools reuse what a stream
 // has freed by waiting for that stream, without asking every live stream how far it is: a batch
@@ -48,6 +48,11 @@ constexpr unsigned long long POOL_KEEP_BYTES = 512ULL << 20;
 constexpr size_t POOL_MOST_BYTES = (size_t) 128 << 20;
 enum class Pool { SCRATCH, HANDLE };
 cudaError_t pool_alloc(void ** p, size_t bytes, Pool pool, cudaStream_t s);
+// Bytes of the HANDLE pool that handles took (or gave back, < 0): its release threshold, which
+// counts memory in use, is kept that far above.  With the bare bound, handles that held more had
+// every synchronisation unmap what was free: 48 conversions beside 3.5 GB of other matrices spent
+// 6.1 ms allocating and 8.0 freeing, 2.4 and 4.9 so.
+void pool_live(int64_t bytes);
 
 // While it lives, memory calls of this thread go through beside a stream capture, its own or
 // another thread's, which they otherwise end.

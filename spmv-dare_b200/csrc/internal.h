@@ -186,6 +186,7 @@ struct Handle {
 	struct Allocation {
 		void * p;
 		bool pooled;
+		int64_t bytes;
 	};
 	std::vector<Allocation> allocations;    // everything above, freed by destroy
 	double mem_footprint = 0;
@@ -213,7 +214,9 @@ struct Handle {
 			set_error(SPMV_ERR_NOMEM, "device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
 			return SPMV_ERR_NOMEM;
 		}
-		allocations.push_back({(void *) *p, pooled});
+		allocations.push_back({(void *) *p, pooled, (int64_t) bytes});
+		if (pooled)
+			pool_live((int64_t) bytes);
 		device_bytes += (int64_t) bytes;
 		return SPMV_OK;
 	}

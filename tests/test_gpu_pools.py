@@ -6,6 +6,9 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
+MB = 1 << 20
+KEEP = 512 * MB          # unused memory a pool keeps
+
 
 def _matrix(r, m):
     lengths = r.integers(0, 30, m)
@@ -35,3 +38,35 @@ def test_conversion_time_does_not_grow_with_the_matrices_alive(sb):
     alive = [sb.Batch(mats, fmts) for _ in range(4)]
     beside = least()
     assert len(alive) == 4 and beside < 2 * alone, (alone, beside)
+
+
+def _device_matrix(torch, entries, m=100000):
+    """Rows of equal length on the GPU: 12 bytes an entry, arrays of less than 128 MB each."""
+    k = entries // m
+    rp = torch.arange(m + 1, dtype=torch.int32, device="cuda") * k
+    ci = torch.arange(k, dtype=torch.int32, device="cuda").repeat(m)
+    return rp, ci, torch.ones(k * m, dtype=torch.float64, device="cuda")
+
+
+def _free(torch):
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+
+
+def test_unused_memory_is_kept_beside_many_matrices(sb):
+    """Matrices that hold more than a pool keeps do not make it give back what is free."""
+    import torch
+
+    big, small = _device_matrix(torch, 10_000_000), _device_matrix(torch, 1_000_000)
+    held = [sb.csr_to_format(*big, format="csr_naive", kernel=4) for _ in range(7)]      # 840 MB of arrays
+    other = sb.csr_to_format(*big, format="csr_naive", kernel=4)
+    before = _free(torch)
+    other.destroy()
+    for _ in range(3):                                   # conversions synchronise
+        sb.csr_to_format(*small, format="csr_naive").destroy()
+    assert _free(torch) - before < 32 * MB               # the 120 MB of `other` wait for the next conversion
+    for h in held:
+        h.destroy()
+    for _ in range(3):
+        sb.csr_to_format(*small, format="csr_naive").destroy()
+    assert _free(torch) - before >= 840 * MB + 120 * MB - KEEP - 64 * MB
