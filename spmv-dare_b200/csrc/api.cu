@@ -82,18 +82,8 @@ static cudaError_t device_pools(DevicePools ** out)
 cudaError_t pool_alloc(void ** p, size_t bytes, Pool kind, cudaStream_t s)
 {
 	DevicePools * d = nullptr;
-	cudaError_t e = device_pools(&d);
-	if (e != cudaSuccess)
-		return e;
-	e = cudaMallocFromPoolAsync(p, bytes, d->pool[(int) kind], s);
-	if (e == cudaErrorMemoryAllocation) {
-		cudaGetLastError();
-		cudaDeviceSynchronize();
-		for (cudaMemPool_t q : d->pool)
-			cudaMemPoolTrimTo(q, 0);
-		e = cudaMallocFromPoolAsync(p, bytes, d->pool[(int) kind], s);
-	}
-	return e;
+	const cudaError_t e = device_pools(&d);
+	return e != cudaSuccess ? e : cudaMallocFromPoolAsync(p, bytes, d->pool[(int) kind], s);
 }
 
 void pool_live(int64_t bytes)

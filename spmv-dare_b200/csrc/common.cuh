@@ -36,8 +36,8 @@ int  last_status();
 // Stream-ordered allocations on the current device, from two pools per device of the library's
 // own: one for scratch, one for the arrays of handles up to POOL_MOST_BYTES each (larger ones are
 // plain allocations).  Mapping and unmapping memory cost a conversion more than its kernels, so
-// each pool keeps up to POOL_KEEP_BYTES that nothing uses; an allocation that
-// fails gives all of it back first and tries again.  (One pool for both, or larger arrays in it,
+// each pool keeps up to POOL_KEEP_BYTES that nothing uses; the driver takes that back by itself
+// when another allocation of the process, in a pool or a plain one, finds no memory.  (One pool for both, or larger arrays in it,
 // put live arrays above the bound, and every synchronisation unmapped the scratch: 34 ms
 // against 12 for a 2M-row SELL conversion.)  A SELL-C-sigma conversion of 8.5 M host entries with
 // one SpMV: 12.8 ms with cudaMalloc and the default pool, 5.9 so.  The pools reuse what a stream

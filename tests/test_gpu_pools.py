@@ -1,4 +1,5 @@
 """The library's memory pools: what they keep between conversions, and what they give back."""
+import threading
 import time
 
 import numpy as np
@@ -70,3 +71,68 @@ def test_unused_memory_is_kept_beside_many_matrices(sb):
     for _ in range(3):
         sb.csr_to_format(*small, format="csr_naive").destroy()
     assert _free(torch) - before >= 840 * MB + 120 * MB - KEEP - 64 * MB
+
+
+class _OnlyFree:
+    """Leaves `left` bytes of the device free while it lives."""
+
+    def __init__(self, torch, left):
+        self.torch, self.left = torch, left
+
+    def __enter__(self):
+        self.torch.cuda.empty_cache()
+        self.fill = self.torch.empty(_free(self.torch) - self.left, dtype=self.torch.uint8, device="cuda")
+
+    def __exit__(self, *exc):
+        del self.fill
+        self.torch.cuda.empty_cache()
+
+
+def test_a_large_array_takes_what_the_pools_keep(sb):
+    """200 MB free and more kept in the pool: a 240 MB array of values still finds its place."""
+    import torch
+
+    csr = _device_matrix(torch, 30_000_000)
+    expect = sb.csr_to_format(*csr, format="csr_naive", kernel=4).spmv(torch.ones(100000, dtype=torch.float64, device="cuda"))
+    x = torch.ones(100000, dtype=torch.float64, device="cuda")
+    y = torch.empty_like(expect)
+    kept = [sb.csr_to_format(*_device_matrix(torch, 10_000_000), format="csr_naive", kernel=4) for _ in range(4)]
+    for h in kept:                                       # 480 MB stay in the pool
+        h.destroy()
+    with _OnlyFree(torch, 200 * MB):
+        h = sb.csr_to_format(*csr, format="csr_naive", kernel=4)
+        h.spmv(x, y)
+        h.destroy()
+    assert torch.equal(y, expect)
+
+def test_an_allocation_without_memory_leaves_captures_alone(sb):
+    """Conversions of another thread until the device is full: refused, and the capture goes on."""
+    import torch
+
+    csr = _device_matrix(torch, 10_000_000)
+    x = torch.ones(100000, dtype=torch.float64, device="cuda")
+    held, status = [], []
+    mf = sb.csr_to_format(*csr, format="csr_naive", kernel=4)
+    expect, y = mf.spmv(x), torch.zeros_like(x)
+
+    def convert():
+        try:
+            while len(held) < 20:
+                held.append(sb.csr_to_format(*csr, format="csr_naive", kernel=4))
+        except sb.SpmvError as e:
+            status.append(e.status)
+
+    with _OnlyFree(torch, 200 * MB):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, capture_error_mode="thread_local"):
+            mf.spmv(x, y)
+            t = threading.Thread(target=convert)
+            t.start()
+            t.join()
+            mf.spmv(x, y)
+        g.replay()
+        torch.cuda.synchronize()
+        for h in held:
+            h.destroy()
+    assert status == [sb._capi.SPMV_ERR_NOMEM]
+    assert torch.equal(y, expect)
