@@ -318,6 +318,11 @@ int spmv_export(const spmv_handle * h, int32_t array_id, void * dst, int64_t * c
 
 void spmv_destroy(spmv_handle * h);
 
+/* Gives the device memory that the library keeps between conversions (at most 512 MB unused in each of
+ * two pools a device) back, on the current device.  Within the process the driver takes it by itself
+ * when an allocation finds no other memory; other processes see it free only after this call. */
+int spmv_release_memory(void);
+
 /* Message of the calling thread's last error ("" if none). */
 const char * spmv_last_error(void);
 

@@ -55,6 +55,13 @@ def _raise(status):
     raise SpmvError(status, msg or "error")
 
 
+def release_memory():
+    """Gives the device memory kept between conversions (unused, at most 1 GB) back, for other processes."""
+    st = library().spmv_release_memory()
+    if st:
+        _raise(st)
+
+
 def format_defaults(format="csr_naive"):
     """The reference's defaults for `format` as a dict of descriptor fields."""
     d = _capi.FormatDesc()

@@ -95,6 +95,7 @@ SIGNATURES = {
     "spmv_get_info": (c_int, [c_void_p, POINTER(Info)]),
     "spmv_export": (c_int, [c_void_p, c_int32, c_void_p, POINTER(c_int64)]),
     "spmv_destroy": (None, [c_void_p]),
+    "spmv_release_memory": (c_int, []),
     "spmv_last_error": (c_char_p, []),
     "spmv_statistics_print_labels": (c_int, [c_char_p, c_int64]),
     "spmv_statistics_print_data": (c_int, [c_void_p, c_char_p, c_int64]),

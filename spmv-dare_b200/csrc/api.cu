@@ -86,6 +86,15 @@ cudaError_t pool_alloc(void ** p, size_t bytes, Pool kind, cudaStream_t s)
 	return e != cudaSuccess ? e : cudaMallocFromPoolAsync(p, bytes, d->pool[(int) kind], s);
 }
 
+cudaError_t pools_trim()
+{
+	DevicePools * d = nullptr;
+	cudaError_t e = device_pools(&d);
+	for (int k = 0; k < 2 && e == cudaSuccess; k++)
+		e = cudaMemPoolTrimTo(d->pool[k], 0);
+	return e;
+}
+
 void pool_live(int64_t bytes)
 {
 	DevicePools * d = nullptr;
@@ -744,6 +753,13 @@ void spmv_destroy(spmv_handle * H)
 		return;
 	spmv::release_handle(H->h);
 	delete H;
+}
+
+int spmv_release_memory(void)
+{
+	spmv::clear_error();
+	SPMV_CUDA_TRY(spmv::pools_trim());
+	return SPMV_OK;
 }
 
 const char * spmv_last_error(void)

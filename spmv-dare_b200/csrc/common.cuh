@@ -53,6 +53,7 @@ cudaError_t pool_alloc(void ** p, size_t bytes, Pool pool, cudaStream_t s);
 // every synchronisation unmap what was free: 48 conversions beside 3.5 GB of other matrices spent
 // 6.1 ms allocating and 8.0 freeing, 2.4 and 4.9 so.
 void pool_live(int64_t bytes);
+cudaError_t pools_trim();      // gives the unused memory of the current device's pools back
 
 // While it lives, memory calls of this thread go through beside a stream capture, its own or
 // another thread's, which they otherwise end.

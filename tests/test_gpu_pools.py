@@ -136,3 +136,17 @@ def test_an_allocation_without_memory_leaves_captures_alone(sb):
             h.destroy()
     assert status == [sb._capi.SPMV_ERR_NOMEM]
     assert torch.equal(y, expect)
+
+
+def test_release_memory(sb):
+    import torch
+
+    csr = _device_matrix(torch, 10_000_000)
+    sb.release_memory()
+    before = _free(torch)
+    held = [sb.csr_to_format(*csr, format="csr_naive", kernel=4) for _ in range(3)]
+    for h in held:
+        h.destroy()
+    assert before - _free(torch) >= 300 * MB             # kept for the next conversions
+    sb.release_memory()
+    assert before - _free(torch) < 32 * MB
