@@ -247,9 +247,12 @@ int build_batch_tiles(spmv_batch * b, int32_t count, const int32_t * const * row
 		int sms = 0;
 		cudaGetDevice(&b->device);
 		cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
-		st = spmv::build_tiles(b->tiles, src, 0, false, true, sms, b->stream, [b](void ** p, size_t bytes) {
-			return balloc(b, (uint8_t **) p, (int64_t) bytes);
-		});
+		st = spmv::build_tiles(b->tiles, src, 0, false, true, sms, b->stream,
+				{[b](void ** p, size_t bytes) { return balloc(b, (uint8_t **) p, (int64_t) bytes); },
+				 [b](void * p) {
+					 cudaFree(p);
+					 b->allocs.erase(std::find(b->allocs.begin(), b->allocs.end(), p));
+				 }});
 	}
 	if (st == SPMV_OK && b->tiles.built) {
 		SPMV_CUDA_TRY(cudaStreamSynchronize(b->stream));

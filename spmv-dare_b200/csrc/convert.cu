@@ -539,7 +539,7 @@ int build_row_tiles(Handle & h)
 	const bool f32 = h.desc.values == SPMV_VALUES_F32;
 	const int lanes = h.desc.format == SPMV_FMT_CSR_VEC && !f32 ? h.desc.vec_len : 0;
 	return build_tiles(h.tiles, {tile_source(h)}, lanes, f32, false, h.num_sms, h.stream,
-			[&h](void ** p, size_t bytes) { return h.alloc((uint8_t **) p, (int64_t) bytes); });
+			{[&h](void ** p, size_t bytes) { return h.alloc((uint8_t **) p, (int64_t) bytes); }, [&h](void * p) { h.drop(p); }});
 }
 
 // Kernel choice: -1 = the format's default (row tiles where tiles_default says so; else the

@@ -220,6 +220,20 @@ struct Handle {
 		device_bytes += (int64_t) bytes;
 		return SPMV_OK;
 	}
+	// Frees one of the allocations, which only work on `stream` used.
+	void drop(void * p)
+	{
+		for (size_t i = 0; i < allocations.size(); i++) {
+			const Allocation a = allocations[i];
+			if (a.p != p)
+				continue;
+			if ((a.pooled ? cudaFreeAsync(p, stream) : cudaFree(p)) == cudaSuccess && a.pooled)
+				pool_live(-a.bytes);
+			device_bytes -= a.bytes;
+			allocations.erase(allocations.begin() + i);
+			return;
+		}
+	}
 };
 
 // ---- conversions (each fills the format's device arrays from d_rp/d_ci/d_v)

@@ -60,10 +60,17 @@ struct TilePlan {
 	int64_t nranges = 0, nlong = 0, grid = 0;
 };
 
-// Builds the layout; p.built stays false where it does not pay (padding above a third of the
-// entries) or does not fit 32-bit indices.  lanes: 4 or 8 for csr_vec's row sums, else 0.
+// Where a layout's arrays live: those of a handle or a batch.
+struct TileMemory {
+	std::function<int(void **, size_t)> take;
+	std::function<void(void *)> drop;        // before the owner's end
+};
+
+// Builds the layout; p.built stays false, and nothing of it stays allocated, where it does not pay
+// (padding above a third of the entries) or does not fit 32-bit indices.  lanes: 4 or 8 for
+// csr_vec's row sums, else 0.
 int build_tiles(TilePlan & p, const std::vector<TileSource> & src, int lanes, bool f32, bool mixed, int num_sms,
-		cudaStream_t s, const std::function<int(void **, size_t)> & alloc);
+		cudaStream_t s, const TileMemory & memory);
 int launch_tiles(const TilePlan & p, const void * x, void * y, cudaStream_t s);
 
 }  // namespace spmv

@@ -890,12 +890,9 @@ TileFn tile_fn(const TilePlan & p)
 	                : tile_kernel<Sum::FMA, DEEP_CTAS, true>;
 }
 
-}  // namespace
-
-int build_tiles(TilePlan & p, const std::vector<TileSource> & src, int lanes, bool f32, bool mixed, int num_sms,
+int lay_out(TilePlan & p, const std::vector<TileSource> & src, int lanes, bool f32, bool mixed, int num_sms,
 		cudaStream_t s, const std::function<int(void **, size_t)> & alloc)
 {
-	p.built = false;
 	p.f32 = f32;
 	p.mixed = mixed;
 	p.lanes = lanes;
@@ -1032,6 +1029,27 @@ int build_tiles(TilePlan & p, const std::vector<TileSource> & src, int lanes, bo
 	p.pad_col = src[0].pad_col;
 	p.built = true;
 	return SPMV_OK;
+}
+
+}  // namespace
+
+int build_tiles(TilePlan & p, const std::vector<TileSource> & src, int lanes, bool f32, bool mixed, int num_sms,
+		cudaStream_t s, const TileMemory & memory)
+{
+	std::vector<void *> taken;
+	p = TilePlan();
+	const int st = lay_out(p, src, lanes, f32, mixed, num_sms, s, [&](void ** a, size_t bytes) {
+		const int got = memory.take(a, bytes);
+		if (got == SPMV_OK)
+			taken.push_back(*a);
+		return got;
+	});
+	if (!p.built) {
+		for (void * a : taken)
+			memory.drop(a);
+		p = TilePlan();
+	}
+	return st;
 }
 
 int launch_tiles(const TilePlan & p, const void * x, void * y, cudaStream_t s)
