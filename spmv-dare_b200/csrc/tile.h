@@ -67,8 +67,9 @@ struct TileMemory {
 };
 
 // Builds the layout; p.built stays false, and nothing of it stays allocated, where it does not pay
-// (padding above a third of the entries) or does not fit 32-bit indices.  lanes: 4 or 8 for
-// csr_vec's row sums, else 0.
+// (padding above a third of the entries), does not fit 32-bit indices or finds no memory (a second
+// copy of the entries, which the staged kernels do without).  lanes: 4 or 8 for csr_vec's row
+// sums, else 0.
 int build_tiles(TilePlan & p, const std::vector<TileSource> & src, int lanes, bool f32, bool mixed, int num_sms,
 		cudaStream_t s, const TileMemory & memory);
 int launch_tiles(const TilePlan & p, const void * x, void * y, cudaStream_t s);

