@@ -316,6 +316,12 @@ int spmv_get_info(const spmv_handle * h, spmv_info * out);
 #define SPMV_ARR_DIV_THREAD_GROUPS 34 /* int64[T]             packet groups per thread           */
 int spmv_export(const spmv_handle * h, int32_t array_id, void * dst, int64_t * count);
 
+/* Which kernel spmv_run* launches: its number among those of spmv_format_desc.kernel, 11 for row
+ * tiles, for DIV-RF 3 for the segment decoder.  variant: row tiles: 1 the build for many ranges a
+ * warp, + 2 the one that fetches a line of x once for rows that share it; segment decoder: warps a
+ * packet, + 64 the build of three CTAs an SM; else 0. */
+int spmv_exec_choice(const spmv_handle * h, int32_t * kernel, int32_t * variant);
+
 void spmv_destroy(spmv_handle * h);
 
 /* Gives the device memory that the library keeps between conversions (at most 512 MB unused in each of
@@ -352,6 +358,8 @@ int spmv_batch_run_graph(spmv_batch * b, const double * d_x, double * d_y, void 
 int spmv_batch_sync(spmv_batch * b);
 int spmv_batch_info(const spmv_batch * b, int64_t * total_x, int64_t * total_y, int64_t * total_nnz,
 		int64_t * x_offsets, int64_t * y_offsets, int64_t * num_blocks);
+/* As spmv_exec_choice: 11 row tiles, 0 the work queue, csr_naive batches their merged matrix's. */
+int spmv_batch_exec_choice(const spmv_batch * b, int32_t * kernel, int32_t * variant);
 void spmv_batch_destroy(spmv_batch * b);
 
 /* ---------------------------------------------------------------- artificial matrices */

@@ -20,7 +20,7 @@ device-resident path, enqueued on torch's current stream).
 from __future__ import annotations
 
 import ctypes
-from ctypes import byref, c_int, c_int64
+from ctypes import byref, c_int, c_int32, c_int64
 
 import numpy as np
 
@@ -236,6 +236,14 @@ class Matrix_Format:
         library().spmv_statistics_print_data(self._h, buf, len(buf))
         return buf.value.decode()
 
+    def exec_choice(self):
+        """(kernel, variant) that spmv() launches, as spmv_exec_choice numbers them."""
+        k, v = c_int32(), c_int32()
+        st = library().spmv_exec_choice(self._h, byref(k), byref(v))
+        if st:
+            _raise(st)
+        return k.value, v.value
+
     def destroy(self):
         if self._h is not None:
             library().spmv_destroy(self._h)
@@ -354,6 +362,14 @@ class Batch:
         st = library().spmv_batch_sync(self._b)
         if st:
             _raise(st)
+
+    def exec_choice(self):
+        """(kernel, variant) that spmv() launches, as spmv_batch_exec_choice numbers them."""
+        k, v = c_int32(), c_int32()
+        st = library().spmv_batch_exec_choice(self._b, byref(k), byref(v))
+        if st:
+            _raise(st)
+        return k.value, v.value
 
     def destroy(self):
         if getattr(self, "_b", None):

@@ -94,6 +94,7 @@ SIGNATURES = {
     "spmv_sync": (c_int, [c_void_p]),
     "spmv_get_info": (c_int, [c_void_p, POINTER(Info)]),
     "spmv_export": (c_int, [c_void_p, c_int32, c_void_p, POINTER(c_int64)]),
+    "spmv_exec_choice": (c_int, [c_void_p, POINTER(c_int32), POINTER(c_int32)]),
     "spmv_destroy": (None, [c_void_p]),
     "spmv_release_memory": (c_int, []),
     "spmv_last_error": (c_char_p, []),
@@ -113,6 +114,7 @@ SIGNATURES = {
     "spmv_batch_run_graph": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p]),
     "spmv_batch_sync": (c_int, [c_void_p]),
     "spmv_batch_info": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),
+    "spmv_batch_exec_choice": (c_int, [c_void_p, POINTER(c_int32), POINTER(c_int32)]),
     "spmv_batch_destroy": (None, [c_void_p]),
     "spmv_mtx_read": (c_void_p, [c_char_p, c_int32, POINTER(c_int)]),
     "spmv_mtx_info": (c_int, [c_void_p] + [c_void_p] * 7),

@@ -755,6 +755,25 @@ void spmv_destroy(spmv_handle * H)
 	delete H;
 }
 
+int spmv_exec_choice(const spmv_handle * H, int32_t * kernel, int32_t * variant)
+{
+	spmv::clear_error();
+	if (!H || !kernel || !variant) {
+		spmv::set_error(SPMV_ERR_ARG, "null handle or result");
+		return SPMV_ERR_ARG;
+	}
+	const Handle & h = H->h;
+	*kernel = h.exec_kernel;
+	*variant = 0;
+	if (h.desc.format == SPMV_FMT_DIV_RF) {
+		if (h.exec_kernel == 3)
+			*variant = h.div_warps + (h.div_warps == 8 && spmv::div_three_ctas(h) ? 64 : 0);
+	} else if (h.exec_kernel == 11) {
+		*variant = (h.tiles.wide ? 1 : 0) + (h.tiles.staged ? 2 : 0);
+	}
+	return SPMV_OK;
+}
+
 int spmv_release_memory(void)
 {
 	spmv::clear_error();

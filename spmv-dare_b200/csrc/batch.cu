@@ -556,6 +556,19 @@ int spmv_batch_info(const spmv_batch * b, int64_t * total_x, int64_t * total_y, 
 	return SPMV_OK;
 }
 
+int spmv_batch_exec_choice(const spmv_batch * b, int32_t * kernel, int32_t * variant)
+{
+	if (!b || !kernel || !variant) {
+		spmv::set_error(SPMV_ERR_ARG, "batch: null argument");
+		return SPMV_ERR_ARG;
+	}
+	if (b->merged)
+		return spmv_exec_choice(b->merged, kernel, variant);
+	*kernel = b->tiles.built ? 11 : 0;
+	*variant = b->tiles.built && b->tiles.wide ? 1 : 0;
+	return SPMV_OK;
+}
+
 void spmv_batch_destroy(spmv_batch * b)
 {
 	if (b)

@@ -1931,6 +1931,11 @@ int convert_div(Handle & h)
 	return SPMV_OK;
 }
 
+bool div_three_ctas(const Handle & h)
+{
+	return h.num_packets <= 3 * h.num_sms;
+}
+
 int launch_div(Handle & h, const double * d_x, double * d_y, cudaStream_t s)
 {
 	if (h.num_packets == 0) {
@@ -1954,9 +1959,8 @@ int launch_div(Handle & h, const double * d_x, double * d_y, cudaStream_t s)
 		g.end = h.d_div + h.div_bytes;
 		g.x = d_x;
 		g.y = d_y;
-		SPMV_CUDA_TRY(launch_overlapped(div_segment_fn(h.desc.vec_len, h.div_warps,
-				h.num_packets <= 3 * h.num_sms), (unsigned) h.num_packets,
-				(unsigned) h.div_warps * 32, 0, s, g));
+		SPMV_CUDA_TRY(launch_overlapped(div_segment_fn(h.desc.vec_len, h.div_warps, div_three_ctas(h)),
+				(unsigned) h.num_packets, (unsigned) h.div_warps * 32, 0, s, g));
 		return SPMV_OK;
 	}
 	DivArgs a;

@@ -259,6 +259,7 @@ int build_tile_reg(Handle & h, const int32_t * d_P, int64_t U, int V);
 bool tiles_default(const Handle & h, int V);  // the descriptor leaves the kernel to the library
 TileSource tile_source(const Handle & h);
 int build_row_tiles(Handle & h);
+bool div_three_ctas(const Handle & h);        // the segment decoder of 8 warps: three CTAs an SM
 int launch_warp(Handle & h, const double * d_x, double * d_y, cudaStream_t s);
 
 // ---- SpMV launches

@@ -19,8 +19,9 @@ def test_a_refused_layout_keeps_no_memory(sb, fmt, kw):
     rp, ci, v, _ = _matrix(lengths, 3)
     args = (rp, ci, v, m, N, int(rp[-1]))
     assert rp[-1] >= THRESHOLD
-    assert sb.csr_to_format(*args, format=fmt, **kw).device_bytes == \
-        sb.csr_to_format(*args, format=fmt, kernel=4, **kw).device_bytes
+    h = sb.csr_to_format(*args, format=fmt, **kw)
+    assert h.exec_choice() == (4, 0)
+    assert h.device_bytes == sb.csr_to_format(*args, format=fmt, kernel=4, **kw).device_bytes
 
 
 # what is left free (MB): the format's arrays of 20 M entries fit, the layout's 240 (FP32: 160) beside them do not
