@@ -999,13 +999,49 @@ __global__ void __launch_bounds__(DIVW_WARPS * 32, MINB) div_warp_kernel(DivArgs
 // 512 or 1,024, 32 lanes 202 and 218.
 // Seven CTAs an SM fit in 72 registers a thread: 8 M entries of 300 values, 2.2 waves of six CTAs
 // 115 us, 1.9 of seven 91; eight spill, 94.
-// Warps a packet (4, 8, 16 or 32, in shorter segments from 8 on): from the waves of mean packets and
+// Warps a packet (4, 8, 16 or 32, in shorter segments from 8 on; fewer than 4 below): from the waves of mean packets and
 // the largest packet, a warp's share of the larger; twice the warps only where that nearly
 // halves, since 64 registers a thread spill (371 packets 30 us with 16 warps, in two waves).  204 packets 110 us with 4 warps, 59 with the CTA
 // decoder, 46 so; 12 packets 59, 30 and 17; 571 packets 43, 43 and 30 with 8 warps; 782 44 with 4
 // and 46 with 8; 1,000 packets, some of long rows and four times the mean, 119, 121 and 74 with 8.
+// Small packets take 2 warps or 1 in CTAs of that many, as many warps an SM as with four: a warp
+// without a segment holds its place for nothing, and each CTA pays a chain of header loads worth
+// 0.4 segments.  Those CTAs have 256 sums (with 512 of them 14 or 28 CTAs leave the L1 too little:
+// 32 lanes, packets of 512 values 791 us, 665 so).  With 32 lanes of more than 1,100 unique values
+// the payload lines of 28 packets a SM crowd each other out of the L1, and four warps that share
+// a packet's stay (2,048 values: 802, 765 and 732 us with 1, 2 and 4).  80 M distinct values in
+// packets of 512 / 1,024 / 2,048: 4 lanes 1,606 / 922 / 777 us with four warps, 803 / 740 / 727
+// now; 32 lanes 2,097 / 1,115 / 732, 665 / 687 / 712 now, 870 / 744 / 712 with the warp decoder.
+// That one keeps packets of 1,100 to 3,600 distinct values in 32 lanes where its warps go round at
+// least 2.5 times: four warps find 3 to 7 segments there (80 M in packets of 2,560 values 826 us,
+// 713 with it; 20 M in packets of 2,048 196 and 189); few values, longer packets and fewer rounds
+// are the segment decoder's (80 M of 300 values, packets of 2,048: 2,624 and 994).
 constexpr int DIVS_CTAS = 7;
 constexpr int DIVS_SUMS = 512;
+constexpr int64_t DIVS_LANE_VALUES = 1100, DIVW_MOST_VALUES = 3600;
+
+bool div_warp_decoder_better(int L, int64_t packets, int64_t entries, int64_t unique, int num_sms)
+{
+	return L == 32 && unique * 10 >= entries * 9 && entries >= DIVS_LANE_VALUES * packets &&
+			entries < DIVW_MOST_VALUES * packets && packets * 2 >= (int64_t) num_sms * 24 * 5;
+}
+
+// 1, 2 or 4, in units of a segment's time: what the SMs' warps take for the mean packet's segments,
+// which w warps share unevenly, and the largest packet alone, half of it after the others.  Fewer
+// than four where that saves a twentieth.
+int div_few_warps(int L, int64_t packets, int64_t entries, int64_t largest, int64_t segments, int64_t unique, int num_sms)
+{
+	if (L == 32 && unique > DIVS_LANE_VALUES * packets)
+		return 4;
+	const double mean = (double) segments / packets, most = (double) segments / entries * largest;
+	auto time = [&](int w) {
+		const double share = mean / w + 0.25 * (w - 1) / w;
+		return (0.4 + (share > 1 ? share : 1)) * packets * w / (num_sms * DIVS_CTAS * 4) +
+				0.45 * (0.4 + (most / w > 1 ? most / w : 1));
+	};
+	const int w = time(2) * 1.05 < time(4) ? 2 : 4;
+	return time(1) * (w == 4 ? 1.05 : 1.0) < time(w) ? 1 : w;
+}
 
 int div_warps_per_packet(int64_t packets, int64_t entries, int64_t largest, int num_sms)
 {
@@ -1131,16 +1167,18 @@ __device__ __forceinline__ void prefetch_l1(const uint8_t * p, const uint8_t * e
 		asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
 }
 
-// Sums a row in a packet of nrows <= DEC_MAX_ROWS rows: a power of two, nrows of them in DIVS_SUMS.
+// Sums a row in a packet of nrows <= DEC_MAX_ROWS rows: a power of two, nrows of them in SUMS.
+template <int SUMS>
 __device__ __forceinline__ uint32_t div_copies(int64_t nrows)
 {
-	return 1u << min(5, 31 - __clz(max(DIVS_SUMS / max((int) nrows, 1), 1)));
+	return 1u << min(5, 31 - __clz(max(SUMS / max((int) nrows, 1), 1)));
 }
 
-template <int L, int WARPS, int CTAS = (WARPS > 4 ? 32 / WARPS : DIVS_CTAS)>
+template <int L, int WARPS, int CTAS = (WARPS > 4 ? 32 / WARPS : DIVS_CTAS * 4 / WARPS)>
 __global__ void __launch_bounds__(WARPS * 32, CTAS) div_segment_kernel(DivSegArgs a)
 {
-	__shared__ double ys[DIVS_SUMS];
+	constexpr int SUMS = WARPS > 2 ? DIVS_SUMS : DEC_MAX_ROWS;
+	__shared__ double ys[SUMS];
 	release_next();
 	const int64_t p = blockIdx.x;
 	const int t = threadIdx.x & 31, l = t & (L - 1);
@@ -1183,9 +1221,9 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS) div_segment_kernel(DivSegArg
 	fetch(s);
 	wait_previous();
 	// several sums a row, each of neighbouring threads
-	const uint32_t copies = div_copies(nrows), copy = t & (copies - 1);
+	const uint32_t copies = div_copies<SUMS>(nrows), copy = t & (copies - 1);
 	auto add = [&](uint32_t row, double v) { atomicAdd(&ys[row * copies + copy], v); };
-	for (uint32_t r = threadIdx.x; r < nrows * copies && r < DIVS_SUMS; r += blockDim.x)
+	for (uint32_t r = threadIdx.x; r < nrows * copies && r < SUMS; r += blockDim.x)
 		ys[r] = 0.0;
 	__syncthreads();
 	while (s < s_end) {
@@ -1288,7 +1326,8 @@ template <int L>
 DivSegFn div_segment_fn(int warps, bool three)
 {
 	return warps == 32 ? div_segment_kernel<L, 32> : warps == 16 ? div_segment_kernel<L, 16>
-	     : warps == 8 ? (three ? div_segment_kernel<L, 8, 3> : div_segment_kernel<L, 8>) : div_segment_kernel<L, 4>;
+	     : warps == 8 ? (three ? div_segment_kernel<L, 8, 3> : div_segment_kernel<L, 8>) : warps == 4 ? div_segment_kernel<L, 4>
+	     : warps == 2 ? div_segment_kernel<L, 2> : div_segment_kernel<L, 1>;
 }
 
 DivSegFn div_segment_fn(int L, int warps, bool three)
@@ -1550,7 +1589,7 @@ int convert_div(Handle & h)
 		set_error(SPMV_ERR_ARG, "DIV-RF: kernel %d unavailable (0, or 2 with vec_len 32)", h.desc.kernel);
 		return SPMV_ERR_ARG;
 	}
-	// nothing asked for, lanes within a warp: the segment decoder
+	// nothing asked for, lanes within a warp: the segment decoder (or 2, once the packets are known)
 	if (h.desc.kernel < 0 && L <= 32 && h.desc.block_nnz == 0 && h.desc.stages == 0 && h.desc.ctas_per_sm == 0)
 		h.exec_kernel = 3;
 	// dropped mantissa bits of the lossy mode (reduce_precision, div_kernels_rf.h:467-510)
@@ -1764,6 +1803,8 @@ int convert_div(Handle & h)
 			u_nb.as<int32_t>(), u_pay.as<uint64_t>(), L, h.d_div);
 	SPMV_CUDA_TRY(cudaGetLastError());
 
+	if (h.exec_kernel == 3 && div_warp_decoder_better(L, NP, nnz, U, h.num_sms))
+		h.exec_kernel = 2;
 	if (h.exec_kernel == 3) {
 		// segments of the decoder, each lane's place and value at their starts
 		DevBuf cnt3, nval3, base3, vbase3;
@@ -1790,6 +1831,8 @@ int convert_div(Handle & h)
 		SPMV_CUDA_TRY(cudaMemcpyAsync(&nseg, base3.as<int64_t>() + G, 8, cudaMemcpyDeviceToHost, s));
 		SPMV_CUDA_TRY(cudaMemcpyAsync(&nvals, vbase3.as<int64_t>() + G, 8, cudaMemcpyDeviceToHost, s));
 		SPMV_CUDA_TRY(cudaStreamSynchronize(s));
+		if (h.div_warps == 4)
+			h.div_warps = div_few_warps(L, NP, nnz, largest, nseg, U, h.num_sms);
 		SPMV_TRY(h.alloc(&h.d_pkt_seg, NP + 1));
 		SPMV_TRY(h.alloc(&h.d_segs, 2 * nseg));
 		SPMV_TRY(h.alloc(&h.d_seg_off, nseg * L));

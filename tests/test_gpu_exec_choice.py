@@ -48,13 +48,14 @@ def test_batches(sb):
 @pytest.mark.parametrize("packets,choice", [(100, 32), (250, 16), (400, 8 + 64), (500, 8), (800, 4)])
 @pytest.mark.parametrize("L", [4, 32])
 def test_warps_a_packet(sb, orc, L, packets, choice):
-    """Packets of 8 rows of 128 distinct values."""
+    """Packets of 8 rows of distinct values, four segments each."""
     r = np.random.default_rng(packets)
+    k = 128 if L == 4 else 256                           # segments of 256 and 512
     m, n = 8 * packets, 3000
-    rp = (np.arange(m + 1) * 128).astype(np.int32)
-    ci = (np.repeat(r.integers(0, n - 128, m), 128) + np.tile(np.arange(128), m)).astype(np.int32)
-    v, x = r.integers(-(1 << 30), 1 << 30, 128 * m) / (1 << 30), r.uniform(-1, 1, n)
-    h = sb.csr_to_format(rp, ci, v, m, n, 128 * m, format="div_rf", vec_len=L, div_packet_vals=1024)
+    rp = (np.arange(m + 1) * k).astype(np.int32)
+    ci = (np.repeat(r.integers(0, n - k, m), k) + np.tile(np.arange(k), m)).astype(np.int32)
+    v, x = r.integers(-(1 << 30), 1 << 30, k * m) / (1 << 30), r.uniform(-1, 1, n)
+    h = sb.csr_to_format(rp, ci, v, m, n, k * m, format="div_rf", vec_len=L, div_packet_vals=8 * k)
     assert h.exec_choice() == (3, choice)
     gold, absy = orc.csr_gold(rp, ci, v, x)
     assert rel_row_error(h.spmv(x, np.full(m, 1.0)), gold, absy) <= 1e-12
