@@ -68,6 +68,7 @@ int balloc(spmv_batch * b, T ** p, int64_t count)
 {
 	cudaError_t e = cudaMalloc((void **) p, (size_t) (count > 0 ? count : 1) * sizeof(T));
 	if (e != cudaSuccess) {
+		cudaGetLastError();
 		spmv::set_error(SPMV_ERR_NOMEM, "batch allocation failed: %s", cudaGetErrorString(e));
 		return SPMV_ERR_NOMEM;
 	}
@@ -136,6 +137,8 @@ int build_merged(spmv_batch * b, int32_t count, const int32_t * const * row_ptrs
 	int * bad = nullptr;
 	int st = SPMV_OK;
 	auto fail = [&](cudaError_t e) {
+		if (e != cudaSuccess)
+			cudaGetLastError();
 		if (e != cudaSuccess && st == SPMV_OK) {
 			spmv::set_error(e == cudaErrorMemoryAllocation ? SPMV_ERR_NOMEM : SPMV_ERR_CUDA, "batch merge: %s",
 					cudaGetErrorString(e));

@@ -19,6 +19,7 @@ int  last_status();
 	do {                                                                                     \
 		cudaError_t _e = (expr);                                                         \
 		if (_e != cudaSuccess) {                                                         \
+			cudaGetLastError();      /* reported here, not by the next launch's check */ \
 			spmv::set_error(_e == cudaErrorMemoryAllocation ? SPMV_ERR_NOMEM : SPMV_ERR_CUDA, \
 				"%s failed: %s (%s:%d)", #expr, cudaGetErrorString(_e), __FILE__, __LINE__); \
 			return spmv::last_status();                                              \

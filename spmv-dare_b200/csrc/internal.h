@@ -211,6 +211,7 @@ struct Handle {
 		alloc_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
 		if (e != cudaSuccess) {
 			*p = nullptr;
+			cudaGetLastError();
 			set_error(SPMV_ERR_NOMEM, "device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
 			return SPMV_ERR_NOMEM;
 		}

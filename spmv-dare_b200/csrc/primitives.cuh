@@ -79,6 +79,7 @@ struct DevBuf {
 		cudaError_t e = pool_alloc(&p, bytes ? bytes : 16, Pool::SCRATCH, stream);
 		if (e != cudaSuccess) {
 			p = nullptr;
+			cudaGetLastError();
 			set_error(SPMV_ERR_NOMEM, "scratch allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
 			return SPMV_ERR_NOMEM;
 		}

@@ -1050,7 +1050,6 @@ int build_tiles(TilePlan & p, const std::vector<TileSource> & src, int lanes, bo
 		p = TilePlan();
 	}
 	if (st == SPMV_ERR_NOMEM) {
-		cudaGetLastError();
 		clear_error();
 		return SPMV_OK;
 	}

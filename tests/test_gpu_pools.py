@@ -150,3 +150,21 @@ def test_release_memory(sb):
     assert before - _free(torch) >= 300 * MB             # kept for the next conversions
     sb.release_memory()
     assert before - _free(torch) < 32 * MB
+
+
+def test_a_refused_conversion_leaves_no_error_behind(sb):
+    """After a conversion without memory the next launches, the library's and torch's, find no error."""
+    import torch
+
+    csr = _device_matrix(torch, 10_000_000)
+    x = torch.ones(100000, dtype=torch.float64, device="cuda")
+    h = sb.csr_to_format(*csr, format="csr_naive", kernel=0)
+    expect, y = h.spmv(x), torch.zeros_like(x)
+    sb.release_memory()
+    with _OnlyFree(torch, 60 * MB):
+        with pytest.raises(sb.SpmvError) as refused:
+            sb.csr_to_format(*csr, format="csr_naive", kernel=0)
+        assert refused.value.status == sb._capi.SPMV_ERR_NOMEM
+        h.spmv(x, y)
+        z = y + 0.0
+    assert torch.equal(z, expect)
