@@ -1805,8 +1805,8 @@ int convert_div(Handle & h)
 
 	if (h.exec_kernel == 3 && div_warp_decoder_better(L, NP, nnz, U, h.num_sms))
 		h.exec_kernel = 2;
-	if (h.exec_kernel == 3) {
-		// segments of the decoder, each lane's place and value at their starts
+	// segments of the decoder, each lane's place and value at their starts
+	auto segments = [&]() -> int {
 		DevBuf cnt3, nval3, base3, vbase3;
 		DevBuf most;
 		int32_t largest = 0;
@@ -1845,6 +1845,18 @@ int convert_div(Handle & h)
 				g_pkt.as<int32_t>(), pk_g0.as<int32_t>(), pk_j.as<int32_t>(), gl_base.as<int64_t>(), S.as<int64_t>(),
 				idx.as<uint32_t>(), val_of.as<uint64_t>(), h.d_segs, h.d_seg_off, h.d_seg_val);
 		SPMV_CUDA_TRY(cudaGetLastError());
+		return SPMV_OK;
+	};
+	if (h.exec_kernel == 3) {
+		const int st = segments();
+		if (st == SPMV_ERR_NOMEM) {             // the other decoders need none of it
+			clear_error();
+			for (void * p : {(void *) h.d_pkt_seg, (void *) h.d_segs, (void *) h.d_seg_off, (void *) h.d_seg_val})
+				h.drop(p);
+			h.exec_kernel = L == 32 ? 2 : 0;
+		} else {
+			SPMV_TRY(st);
+		}
 	}
 
 	// 9) packet groups per reference thread (export) and thread byte counts

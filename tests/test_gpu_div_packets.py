@@ -6,6 +6,7 @@ import pytest
 
 from conftest import rel_row_error
 from test_gpu_div_segments import TOL, _values
+from test_gpu_pools import MB, _OnlyFree
 
 pytestmark = pytest.mark.gpu
 
@@ -74,3 +75,39 @@ def test_small_packets_are_no_slower_than_on_the_warp_decoder(sb, packet):
         times.append(best)
         h.destroy()
     assert times[0] <= 1.15 * times[1], times
+
+
+@pytest.mark.parametrize("L,other", [(32, 2), (4, 0)])
+def test_a_matrix_without_room_for_the_segments(sb, L, other):
+    """Where the conversion fits for the decoder without segment tables, it fits for the default."""
+    import torch
+
+    m = 200000
+    rp, ci, v, x = _matrix(m, 20, m, "few", np.random.default_rng(L))
+    csr = [torch.from_numpy(a).cuda() for a in (rp, ci, v)]
+    xd = torch.from_numpy(x).cuda()
+    kw = dict(format="div_rf", vec_len=L, div_packet_vals=64)
+    roomy = sb.csr_to_format(*csr, **kw)
+    assert roomy.exec_choice()[0] == SEGMENTS
+    roomy.destroy()
+    named = sb.csr_to_format(*csr, kernel=other, **kw)
+    expect, y = named.spmv(xd), torch.zeros_like(xd)
+    torch.cuda.synchronize()
+    named.destroy()
+    for left in range(96, 1600, 32):
+        sb.release_memory()
+        with _OnlyFree(torch, left * MB):
+            try:
+                sb.csr_to_format(*csr, kernel=other, **kw).destroy()
+            except sb.SpmvError as e:
+                assert e.status == sb._capi.SPMV_ERR_NOMEM
+                continue
+            sb.release_memory()
+            h = sb.csr_to_format(*csr, **kw)
+            choice = h.exec_choice()
+            h.spmv(xd, y)
+            h.destroy()
+            sb.release_memory()
+            break
+    assert choice == (other, 0)
+    assert torch.allclose(y, expect, rtol=1e-12, atol=1e-12)
