@@ -250,7 +250,7 @@ int build_batch_tiles(spmv_batch * b, int32_t count, const int32_t * const * row
 		int sms = 0;
 		cudaGetDevice(&b->device);
 		cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
-		st = spmv::build_tiles(b->tiles, src, 0, false, true, sms, b->stream,
+		st = spmv::build_tiles(b->tiles, src, 0, false, true, nullptr, sms, b->stream,
 				{[b](void ** p, size_t bytes) { return balloc(b, (uint8_t **) p, (int64_t) bytes); },
 				 [b](void * p) {
 					 cudaFree(p);

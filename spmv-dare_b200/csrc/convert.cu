@@ -480,8 +480,9 @@ static int build_tiled_cols(Handle & h, const int32_t * d_P, int64_t U, int V)
 // 57 8.0 and 9.6; from 7.6 M entries on row tiles are the faster (csr_naive 25.9 and 25.1 us
 // there, 50.4 and 37.0 with 10.7 M; sell_sorted 23.9 and 19.3 with 4.1 M).  The FP32
 // variant: 14.7 and 18.9 us with 2.6 M entries, 24.0 and 23.2 with 4.7 M, 108 and 68 with 24 M
-// scattered ones, 167 and 161 on the 4M-row matrix.  SELL-C-sigma gains at every size: its other
-// kernels give a slice to a warp or two (1,671 rows 18.9 and 3.6 us).
+// scattered ones, 167 and 161 on the 4M-row matrix.  SELL-C-sigma has no such line: uneven rows gain
+// at every size (1,500 rows of 45, the longest 2,300: 18.9 us and 8.4), and where kernel 4 takes less,
+// as for any format with few long rows, staged_time() shows it.
 constexpr int64_t TILE_ENTRIES = 3500000;
 
 bool tiles_default(const Handle & h, int V)
@@ -534,17 +535,37 @@ TileSource tile_source(const Handle & h)
 	return t;
 }
 
+// The kernel that runs without row tiles, measured over 20,000 to 400,000 rows of 45 to 600 entries, even
+// and uneven (ps an entry, csr_naive 2.8 at 45, 3.3 at 100, 5 at 200, 9.5 at 600 entries a row; SELL's
+// padded entries count).  csr_vec sums a row longer than its blocks in one thread a lane.  SELL-C-sigma
+// runs kernel 4, a thread a row, up to C = 64; wider slices have no faster kernel at any size.
+static const StagedTime * staged_time(const Handle & h)
+{
+	static const StagedTime naive{2.3, 70, 8.5, 1, 6.5, 0}, vec4{3.4, 80, 8.5, 1.2, 190, 1280}, vec8{4.4, 62, 12, 1.2, 230, 1280},
+			sell{2.4, 50, 6, 1, 6.5, 0}, sorted{3.4, 65, 6.5, 1.2, 6.5, 0}, f32{2, 60, 9.6, 1.7, 13, 0},
+			sellcs32{3.9, 1e9, 9, 1, 26, 0}, sellcs64{3.9, 1e9, 9, 1, 46, 0};
+	if (h.desc.values == SPMV_VALUES_F32)
+		return &f32;
+	switch (h.desc.format) {
+	case SPMV_FMT_CSR_NAIVE: return &naive;
+	case SPMV_FMT_CSR_VEC: return h.desc.vec_len == 8 ? &vec8 : &vec4;
+	case SPMV_FMT_SELL: return &sell;
+	case SPMV_FMT_SELL_SORTED: return &sorted;
+	default: return h.desc.sellcs_c <= 32 ? &sellcs32 : h.desc.sellcs_c <= 64 ? &sellcs64 : nullptr;
+	}
+}
+
 int build_row_tiles(Handle & h)
 {
 	const bool f32 = h.desc.values == SPMV_VALUES_F32;
 	const int lanes = h.desc.format == SPMV_FMT_CSR_VEC && !f32 ? h.desc.vec_len : 0;
-	return build_tiles(h.tiles, {tile_source(h)}, lanes, f32, false, h.num_sms, h.stream,
+	return build_tiles(h.tiles, {tile_source(h)}, lanes, f32, false, staged_time(h), h.num_sms, h.stream,
 			{[&h](void ** p, size_t bytes) { return h.alloc((uint8_t **) p, (int64_t) bytes); }, [&h](void * p) { h.drop(p); }});
 }
 
-// Kernel choice: -1 = the format's default (row tiles where tiles_default says so; else the
-// register-tiled warp kernel for slices of 32 rows, the tiled warp-specialised kernel for wider
-// SELL-C-sigma slices, the warp-specialised kernel otherwise); 0 = CTA
+// Kernel choice: -1 = the format's default (row tiles where tiles_default says so and the staged
+// kernel would take longer; else the register-tiled warp kernel for slices of 32 rows, the tiled
+// warp-specialised kernel for wider SELL-C-sigma slices, the warp-specialised kernel otherwise); 0 = CTA
 // staged kernel; 1 = direct column-major kernel (slices of >= 32 rows only); 2 =
 // warp-autonomous staged kernel (slices of <= 32 rows); 3 = CTA staged kernel with the next
 // block's gather overlapping this block's rows; 4 = warp-specialised staged kernel; 5 = CTA
@@ -574,7 +595,9 @@ int build_exec(Handle & h, const int32_t * d_P, int64_t U, int V)
 		// block selects the staged kernels.
 		const bool sliced = h.desc.format == SPMV_FMT_SELL_C_S || h.desc.format == SPMV_FMT_SELL ||
 				h.desc.format == SPMV_FMT_SELL_SORTED;
-		if (sliced && V == 32 && h.desc.block_nnz == 0)
+		if (h.tiles.slower && V <= 64)
+			k = 4;                  // what the row tiles were compared with
+		else if (sliced && V == 32 && h.desc.block_nnz == 0)
 			k = 10;
 		else
 			k = h.desc.format == SPMV_FMT_SELL_C_S ? 8 : 4;

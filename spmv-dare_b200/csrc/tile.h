@@ -43,8 +43,17 @@ struct LongUnit {
 	int32_t padded, pad_col;     // the row ends in padding; its column (PAD_OWN: that of the last entry)
 };
 
+// What the staged kernel that would run instead takes, beside a launch: its stored entries, each
+// `base` + (mean row length) / `per_length` ps, at most `most`, times `uneven` where the widest
+// slice is over twice the mean; or its longest row, from `chain_from` entries on, at `chain` ns an entry.
+struct StagedTime {
+	double base, per_length, most, uneven, chain;
+	int chain_from;
+};
+
 struct TilePlan {
 	bool built = false;
+	bool slower = false;         // not built: the staged kernel takes less time
 	int32_t pad_col = PAD_OWN;
 	bool f32 = false, mixed = false, wide = false, staged = false;
 	bool split = false;          // csr_naive arithmetic (MIXED batches: by slice)
@@ -67,11 +76,11 @@ struct TileMemory {
 };
 
 // Builds the layout; p.built stays false, and nothing of it stays allocated, where it does not pay
-// (padding above a third of the entries), does not fit 32-bit indices or finds no memory (a second
-// copy of the entries, which the staged kernels do without).  lanes: 4 or 8 for csr_vec's row
-// sums, else 0.
-int build_tiles(TilePlan & p, const std::vector<TileSource> & src, int lanes, bool f32, bool mixed, int num_sms,
-		cudaStream_t s, const TileMemory & memory);
+// (padding above a third of the entries, rows too few and long for its warps), does not fit 32-bit
+// indices or finds no memory (a second copy of the entries, which the staged kernels do without).
+// lanes: 4 or 8 for csr_vec's row sums, else 0.  staged: the alternative, null: none.
+int build_tiles(TilePlan & p, const std::vector<TileSource> & src, int lanes, bool f32, bool mixed,
+		const StagedTime * staged, int num_sms, cudaStream_t s, const TileMemory & memory);
 int launch_tiles(const TilePlan & p, const void * x, void * y, cudaStream_t s);
 
 }  // namespace spmv

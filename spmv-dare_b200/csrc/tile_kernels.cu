@@ -32,6 +32,8 @@
 // Rows too long for that (a lane would walk them for tens of microseconds) stay in the
 // format's arrays: the first warp of a CTA takes one, its 32 lanes load and gather 256 entries
 // ahead and one lane (csr_vec: one per lane of its order) sums them from shared memory.
+#include <algorithm>
+
 #include "internal.h"
 #include "primitives.cuh"
 #include "tile.h"
@@ -663,28 +665,51 @@ __device__ __forceinline__ bool source_row(const TileSource & s, int64_t i, int6
 	return padded;
 }
 
+// What the sort notes about the rows, beside the number of long ones: the next long row's place, the
+// longest row, the widest slice, and lines of x in the first entries of every eighth window's rows.
+enum { NEXT = 1, LONGEST, WIDEST, LINES, LINES_OF, STATS };
+
 // One CTA per window: its rows sorted by count (descending, stable; long rows and the places
 // past the matrix last), their slots written, and the width of every slice.  A bitonic sort of
 // 1,024 keys in shared memory; key = (max - count) << 10 | place.
 __global__ void __launch_bounds__(TILE_WINDOW / 2) tile_sort_kernel(TileSource s, int long_min, int64_t slot0,
-		int64_t nslots, int32_t * slot_src, int32_t * slot_row, int32_t * slot_cnt, int64_t * width, int * nlong)
+		int64_t nslots, int32_t * slot_src, int32_t * slot_row, int32_t * slot_cnt, int64_t * width, int * stat)
 {
 	__shared__ uint32_t key[TILE_WINDOW];
 	const int64_t base = (int64_t) blockIdx.x * TILE_WINDOW;
 	constexpr uint32_t MOST = (1u << 21) - 1;
 	for (int i = threadIdx.x; i < TILE_WINDOW; i += blockDim.x) {
 		uint32_t rank = MOST;                         // nothing to sum here
+		int64_t start;
+		int stride, cnt = 0;
 		if (base + i < s.m) {
-			int64_t start;
-			int stride, cnt;
 			source_row(s, base + i, start, stride, cnt);
 			if (cnt >= long_min) {
-				atomicAdd(nlong, 1);
+				atomicAdd(&stat[0], 1);
 			} else {
 				rank = MOST - 1 - (uint32_t) cnt;
 			}
 		}
 		key[i] = rank << 10 | (uint32_t) i;
+		const int most = __reduce_max_sync(0xffffffffu, cnt);        // TILE_WINDOW: whole warps
+		if ((i & 31) == 0 && most > *(volatile int *) &stat[LONGEST])
+			atomicMax(&stat[LONGEST], most);
+		// lines of x at the start of some rows
+		if (blockIdx.x % 8 == 0) {
+			const int seen = cnt < 8 ? cnt : 8;
+			int lines = seen > 0, line = seen > 0 ? s.cols[start] >> 4 : 0;
+			for (int k = 1; k < seen; k++) {
+				const int at = s.cols[start + (int64_t) k * stride] >> 4;
+				lines += at != line;
+				line = at;
+			}
+			lines = __reduce_add_sync(0xffffffffu, lines);
+			const int of = __reduce_add_sync(0xffffffffu, seen);
+			if ((i & 31) == 0) {
+				atomicAdd(&stat[LINES], lines);
+				atomicAdd(&stat[LINES_OF], of);
+			}
+		}
 	}
 	for (int size = 2; size <= TILE_WINDOW; size <<= 1)
 		for (int step = size >> 1; step > 0; step >>= 1) {
@@ -713,6 +738,8 @@ __global__ void __launch_bounds__(TILE_WINDOW / 2) tile_sort_kernel(TileSource s
 		slot_cnt[slot] = rank != MOST && source_row(s, r, start, stride, own) ? cnt | PADDED : cnt;
 		if (i % 32 == 0)
 			width[slot / 32] = (int64_t) cnt * 32;
+		if (i == 0)
+			atomicMax(&stat[WIDEST], cnt);
 	}
 }
 
@@ -890,8 +917,35 @@ TileFn tile_fn(const TilePlan & p)
 	                : tile_kernel<Sum::FMA, DEEP_CTAS, true>;
 }
 
-int lay_out(TilePlan & p, const std::vector<TileSource> & src, int lanes, bool f32, bool mixed, int num_sms,
-		cudaStream_t s, const std::function<int(void **, size_t)> & alloc)
+// Whether the staged kernel takes less time.  Row tiles give a slice of 32 rows to a warp, which
+// waits for x tile by tile; below two slices a resident warp (190,000 rows on 148 SMs) the widest
+// slices are their time, and matrices of few long rows took up to eight times as long as on kernel 4
+// (2,000 rows of 2,000, SELL 35 us and 282; csr_naive 6,000 rows of 600 39 and 94, 40,000 of 100 18
+// and 26).  us an entry of the mean and of the widest slice by the slices an SM has: measured 0.14,
+// 0.18 and 0.23 with 1, 4 and 10 or more of even rows of 0.4 lines an entry, half of that with
+// consecutive columns; 0.08 to 0.14 where a few are widest.
+bool staged_takes_less(const StagedTime & k, bool f32, int64_t entries, int64_t rows, int64_t stored, int64_t slices,
+		const int * stat, int num_sms)
+{
+	const int longest = stat[LONGEST], widest = stat[WIDEST];
+	if (slices >= (int64_t) num_sms * 2 * DEEP_CTAS * TILE_WARPS)
+		return false;
+	const double mean = (double) entries / rows, slice = (double) stored / (32 * slices), an_sm = (double) slices / num_sms;
+	const double lines = std::min(1.0, 0.35 + 1.66 * stat[LINES] / std::max(stat[LINES_OF], 1));
+	const double even = lines * std::min(0.13 + 0.012 * an_sm, 0.23), few = lines * std::min(0.08 + 0.004 * an_sm, 0.13);
+	double tiles = stored * (f32 ? 1.6e-6 : 2.4e-6);
+	tiles = std::max(tiles, std::max(slice * even, widest * few));
+	tiles = std::max(tiles, longest * 0.005);
+	double staged = entries * 1e-6 * std::min(k.base + mean / k.per_length, k.most);
+	if (widest > 2 * slice)
+		staged *= k.uneven;
+	if (longest > k.chain_from)
+		staged = std::max(staged, longest * k.chain * 1e-3);
+	return staged < 0.95 * tiles;
+}
+
+int lay_out(TilePlan & p, const std::vector<TileSource> & src, int lanes, bool f32, bool mixed, const StagedTime * staged,
+		int num_sms, cudaStream_t s, const std::function<int(void **, size_t)> & alloc)
 {
 	p.f32 = f32;
 	p.mixed = mixed;
@@ -917,8 +971,8 @@ int lay_out(TilePlan & p, const std::vector<TileSource> & src, int lanes, bool f
 	// 1,830: 112 us with 192 entries and four rows a unit, 66 so).  Shorter ones wait for their
 	// longest rows alone: as many long rows as the chip holds warps beside the slices.
 	DevBuf cnt;
-	SPMV_TRY(cnt.alloc((2 + CENSUS) * sizeof(int), s));
-	SPMV_CUDA_TRY(cudaMemsetAsync(cnt.p, 0, (2 + CENSUS) * sizeof(int), s));
+	SPMV_TRY(cnt.alloc((STATS + CENSUS) * sizeof(int), s));
+	SPMV_CUDA_TRY(cudaMemsetAsync(cnt.p, 0, (STATS + CENSUS) * sizeof(int), s));
 	const int64_t us = 4 + entries * 12 / 6000000;
 	int64_t lm = 2 * us < 512 ? 2 * us : 512;
 	lm = lm > 4 * mean ? lm : 4 * mean;
@@ -927,10 +981,10 @@ int lay_out(TilePlan & p, const std::vector<TileSource> & src, int lanes, bool f
 		int census[CENSUS];
 		for (const TileSource & t : src) {
 			if (t.m > 0)
-				long_census_kernel<<<(unsigned) ceil_div(t.m, 256), 256, 0, s>>>(t, mean, cnt.as<int>() + 2);
+				long_census_kernel<<<(unsigned) ceil_div(t.m, 256), 256, 0, s>>>(t, mean, cnt.as<int>() + STATS);
 			SPMV_CUDA_TRY(cudaGetLastError());
 		}
-		SPMV_CUDA_TRY(cudaMemcpyAsync(census, cnt.as<int>() + 2, sizeof(census), cudaMemcpyDeviceToHost, s));
+		SPMV_CUDA_TRY(cudaMemcpyAsync(census, cnt.as<int>() + STATS, sizeof(census), cudaMemcpyDeviceToHost, s));
 		SPMV_CUDA_TRY(cudaStreamSynchronize(s));
 		for (int i = 0; i < CENSUS; i++)
 			if (census[i] + ns <= (int64_t) num_sms * DEEP_CTAS * TILE_WARPS) {
@@ -961,11 +1015,15 @@ int lay_out(TilePlan & p, const std::vector<TileSource> & src, int lanes, bool f
 	}
 	SPMV_TRY(scan_exclusive(width.as<int64_t>(), sptr64.as<int64_t>(), ns, s));
 	int64_t total = 0;
-	int nlong = 0;
+	int stat[STATS];
 	SPMV_CUDA_TRY(cudaMemcpyAsync(&total, sptr64.as<int64_t>() + ns, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-	SPMV_CUDA_TRY(cudaMemcpyAsync(&nlong, cnt.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+	SPMV_CUDA_TRY(cudaMemcpyAsync(stat, cnt.p, sizeof(stat), cudaMemcpyDeviceToHost, s));
 	SPMV_CUDA_TRY(cudaStreamSynchronize(s));
+	const int nlong = stat[0];
 	if (total > INT32_MAX - 4096 || total > entries + entries / 3 + 65536)
+		return SPMV_OK;
+	p.slower = staged && staged_takes_less(*staged, f32, entries, rows, total, ns, stat, num_sms);
+	if (p.slower)
 		return SPMV_OK;
 	const size_t vs = f32 ? sizeof(float) : sizeof(double);
 	SPMV_TRY(alloc((void **) &p.sptr, (ns + 1) * sizeof(int32_t)));
@@ -986,12 +1044,12 @@ int lay_out(TilePlan & p, const std::vector<TileSource> & src, int lanes, bool f
 			tile_fill_kernel<float><<<g, 256, 0, s>>>(src[i], slot0[i] / 32, n, d_src.as<int32_t>(), p.sptr, p.tcols,
 					(float *) p.vals, p.pad);
 			if (nlong > 0)
-				long_units_kernel<float><<<gl, 256, 0, s>>>(src[i], src[i].vals_f, long_min[i], cnt.as<int>() + 1, p.longs);
+				long_units_kernel<float><<<gl, 256, 0, s>>>(src[i], src[i].vals_f, long_min[i], cnt.as<int>() + NEXT, p.longs);
 		} else {
 			tile_fill_kernel<double><<<g, 256, 0, s>>>(src[i], slot0[i] / 32, n, d_src.as<int32_t>(), p.sptr, p.tcols,
 					(double *) p.vals, p.pad);
 			if (nlong > 0)
-				long_units_kernel<double><<<gl, 256, 0, s>>>(src[i], src[i].vals, long_min[i], cnt.as<int>() + 1, p.longs);
+				long_units_kernel<double><<<gl, 256, 0, s>>>(src[i], src[i].vals, long_min[i], cnt.as<int>() + NEXT, p.longs);
 		}
 		SPMV_CUDA_TRY(cudaGetLastError());
 	}
@@ -1033,12 +1091,12 @@ int lay_out(TilePlan & p, const std::vector<TileSource> & src, int lanes, bool f
 
 }  // namespace
 
-int build_tiles(TilePlan & p, const std::vector<TileSource> & src, int lanes, bool f32, bool mixed, int num_sms,
-		cudaStream_t s, const TileMemory & memory)
+int build_tiles(TilePlan & p, const std::vector<TileSource> & src, int lanes, bool f32, bool mixed,
+		const StagedTime * staged, int num_sms, cudaStream_t s, const TileMemory & memory)
 {
 	std::vector<void *> taken;
 	p = TilePlan();
-	const int st = lay_out(p, src, lanes, f32, mixed, num_sms, s, [&](void ** a, size_t bytes) {
+	const int st = lay_out(p, src, lanes, f32, mixed, staged, num_sms, s, [&](void ** a, size_t bytes) {
 		const int got = memory.take(a, bytes);
 		if (got == SPMV_OK)
 			taken.push_back(*a);
@@ -1047,7 +1105,9 @@ int build_tiles(TilePlan & p, const std::vector<TileSource> & src, int lanes, bo
 	if (!p.built) {
 		for (void * a : taken)
 			memory.drop(a);
+		const bool slower = p.slower;
 		p = TilePlan();
+		p.slower = slower;
 	}
 	if (st == SPMV_ERR_NOMEM) {
 		clear_error();
