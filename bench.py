@@ -23,7 +23,7 @@ from its sources (oracle/_ref), on all host cores.
 log-uniform in [1e3, 2e5], parameters from spmv-dare_b200/workloads.py), each in the format
 the batch autotuner picked for it from the matrices' exhaustive timings
 (spmv-dare_b200/data/tune_batch.npz, tuning.batch_plan; --retune re-runs the timings here).  A step is one SpMV of every matrix: one CUDA-graph replay of
-the persistent work-queue kernel (`value`), beside the same batch launched directly and the
+the batch's launch (`value`), beside the same batch launched directly and the
 512 matrices launched one by one with their own handles.  Metric: the aggregate algorithmic
 bytes of the 512 SpMVs over the step time.
 """
@@ -448,7 +448,7 @@ def tuned_legs(sb, torch, dev, rp, ci, v, x, per_format, B, peak, args):
 
 def mixed_classes(count):
     """Batch formats dealt round robin over sell, sell_sorted, sell_c_s (C=32, sigma=512) and
-    csr_naive: a batch that runs the persistent work-queue kernel."""
+    csr_naive: a batch that runs one launch over all matrices' row tiles."""
     from spmv_dare_b200 import tuning
 
     pool = [tuning.CLASSES.index({"format": "sell", "vec_len": 4}),
@@ -457,11 +457,17 @@ def mixed_classes(count):
     return [pool[i % 4] for i in range(count)]
 
 
+def batch_path(batch, all_csr):
+    kernel = batch.exec_choice()[0]
+    kernel = {11: "row tiles", 4: "warp-specialised kernel", 0: "persistent work-queue batch_kernel"}.get(kernel, f"kernel {kernel}")
+    return f"block-diagonal csr_naive SpMV ({kernel})" if all_csr else kernel
+
+
 def batch_block(sb, torch, dev, args, world, peak):
     """The 512-matrix batch (C4) inside the default line: the autotuned batch (every matrix
     csr_naive with these kernels: one block-diagonal SpMV, CUDA-graph replay) and the same
     matrices with formats dealt round robin over csr_naive / sell / sell_sorted / sell_c_s,
-    which runs the persistent work-queue kernel; y of each against the matrices' own
+    which runs one launch over all matrices' row tiles; y of each against the matrices' own
     handles, bit for bit."""
     from spmv_dare_b200 import tuning
 
@@ -496,8 +502,7 @@ def batch_block(sb, torch, dev, args, world, peak):
             counts[tuning.class_name(c)] = counts.get(tuning.class_name(c), 0) + 1
         out[name] = {"graph_ms": round(ms, 4), "gbs": round(world * B * 1e-9 / (ms * 1e-3), 1),
                      "hbm_frac": round(B * 1e-9 / (med * 1e-3) / peak, 4), "formats": counts,
-                     "path": "block-diagonal csr_naive SpMV (warp-specialised kernel)" if batch.num_blocks == 0 or
-                     all(tuning.CLASSES[c]["format"] == "csr_naive" for c in cls) else "persistent work-queue batch_kernel",
+                     "path": batch_path(batch, all(tuning.CLASSES[c]["format"] == "csr_naive" for c in cls)),
                      "y_identical_to_per_matrix": ident, "steps": steps}
         batch.destroy()
         del yd

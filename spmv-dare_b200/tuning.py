@@ -32,7 +32,7 @@ def _cta(threads, block):
 # BATCHABLE, below: the others repeat earlier descriptors, or the batch engine does not run
 # the format).
 CLASSES = [
-    _ws(160, 64, 768, 3),          # the csr_naive default
+    _ws(160, 64, 768, 3),          # kernel 4's default
     _ws(160, 64, 256, 4),
     _ws(160, 64, 512, 3),
     _ws(192, 64, 1024, 3),
@@ -64,7 +64,10 @@ CLASSES = [
     {"format": "sell", "vec_len": 32, "kernel": 10},
     {"format": "div_rf", "vec_len": 32},
 ]
-DEFAULT_CLASS = 0      # what the library picks without a selector
+# csr_naive on kernel 4: what the library runs without a selector below 3.5 M entries.  Above, its default
+# is row tiles, which no class names (nor SELL-C-sigma's default): the classes and the databases' times
+# stand for the kernels they were measured with.
+DEFAULT_CLASS = 0
 
 
 def batch_desc(i):
@@ -85,8 +88,8 @@ def batch_plan(times, tol=0.05):
     """Per-matrix classes of a batch from its matrices' exhaustive timings (times[i][k], ms):
     csr_naive (the default class) for every matrix when the sum of its times is within `tol`
     of the per-matrix best sum, since an all-csr_naive batch runs as one block-diagonal
-    SpMV on the warp-specialised kernel, about twice the throughput of the mixed-format
-    work queue; otherwise each matrix's own best class."""
+    SpMV of one handle (512 matrices 1.317 ms, with formats in turn on one row-tile layout
+    1.358); otherwise each matrix's own best class."""
     t = np.where(np.isfinite(times), times, np.inf)
     best = np.argmin(t, axis=1)
     if np.sum(t[:, DEFAULT_CLASS]) <= (1.0 + tol) * np.sum(t[np.arange(t.shape[0]), best]):
