@@ -215,7 +215,7 @@ __device__ __forceinline__ T ldg(const T * p)
 // Every CTA calls wait_previous(), so a kernel never ends before the one it overlapped.
 // What it saves is the launch gap and the chain of table loads at a kernel's start: in a loop,
 // csr_naive with 2,000 rows 8.2 -> 6.1 us a pass, with 100,000 8.2 -> 6.5, with 4M 200 -> 191,
-// csr_vec 1M rows 95.3 -> 92.6, sell_sorted 700k rows 65.3 -> 61.4, FP32 4M rows 168 -> 161.
+// csr_vec 1M rows 95.3 -> 92.6, sell_sorted 700k rows 65.3 -> 61.4, FP32 4M rows 168 -> 161-165.
 __device__ __forceinline__ void release_next()
 {
 	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
