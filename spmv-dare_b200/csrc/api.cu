@@ -104,6 +104,21 @@ void pool_live(int64_t bytes)
 	cudaMemPoolSetAttribute(d->pool[(int) Pool::HANDLE], cudaMemPoolAttrReleaseThreshold, &keep);
 }
 
+bool overlaps_last(cudaStream_t s, bool staged, bool few)
+{
+	struct Last {
+		cudaStream_t s;
+		bool any, staged, few;
+	};
+	static thread_local Last last[16];
+	Last & l = last[((uintptr_t) s ^ (uintptr_t) s >> 4 ^ (uintptr_t) s >> 12) & 15];
+	const bool yes = l.any && l.s == s && (l.staged == staged || l.few || few);
+	// few CTAs that overlapped the one before them leave it the last: it may still run
+	if (!(yes && few))
+		l = {s, true, staged, few};
+	return yes;
+}
+
 static const char * kNames[SPMV_NUM_FORMATS] = {
 	"Naive_CSR_B200", "Custom_CSR_VEC_B200", "SELL_B200", "SELL_SORTED_B200", "SELL_C_s_B200", "DIV_RF_B200",
 };

@@ -229,12 +229,21 @@ __device__ __forceinline__ T load_x(const T * p)
 {
 	return __ldca(p);
 }
+// An SM divides its memory between L1 and shared memory when it is idle.  Overlapped, the kernels that
+// want much shared memory (the staged ones: their ring is dynamic) and those that want the L1 (row
+// tiles, DIV-RF) would run on each other's division: SELL on 1 M rows and SELL-C-sigma on 40,000 in turn
+// 82 us apart, 152 overlapped.  So a kernel overlaps one of its own kind, or where either has too few CTAs to
+// matter: overlaps_last() notes the calling thread's last launch on a stream (a hint: what others launch there
+// in between costs time, not results).
+constexpr unsigned FEW_CTAS = 64;
+bool overlaps_last(cudaStream_t s, bool staged, bool few);
 template <typename A>
 cudaError_t launch_overlapped(void (*kernel)(A), unsigned grid, unsigned threads, size_t smem, cudaStream_t s, const A & args)
 {
+	const bool overlap = overlaps_last(s, smem > 0, grid <= FEW_CTAS);
 	cudaLaunchAttribute attr{};
 	attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-	attr.val.programmaticStreamSerializationAllowed = 1;
+	attr.val.programmaticStreamSerializationAllowed = overlap;
 	cudaLaunchConfig_t cfg{};
 	cfg.gridDim = dim3(grid);
 	cfg.blockDim = dim3(threads);

@@ -18,6 +18,41 @@ def _per_step(torch, steps, step):
     return best
 
 
+def _handle(sb, torch, rows, width, fmt, **kw):
+    """Even rows with columns far apart; an SpMV to call."""
+    r = np.random.default_rng(rows)
+    rp = (np.arange(rows + 1) * width).astype(np.int32)
+    ci = (r.integers(0, rows - 8 * width, rows)[:, None] + 8 * np.arange(width)).astype(np.int32).ravel()
+    h = sb.csr_to_format(rp, ci, r.uniform(-1, 1, rows * width), format=fmt, **kw)
+    x = torch.rand(rows, dtype=torch.float32 if "value_type" in kw else torch.float64, device="cuda")
+    y = torch.empty_like(x)
+    return h, lambda: h.spmv(x, y)
+
+
+TILES, STAGED, FEW = (300000, 24, "sell", dict(vec_len=4)), (40000, 45, "sell_c_s", {}), (2000, 20, "csr_naive", {})
+FP32, DIV = (100000, 20, "csr_naive", dict(value_type="f32")), (100000, 24, "div_rf", {})
+
+
+@pytest.mark.parametrize("order", [(TILES, STAGED), (TILES, FP32), (STAGED, DIV), (TILES, FEW), (TILES, FEW, STAGED), (STAGED, FEW, FEW, TILES)])
+def test_kernels_by_turns(sb, order):
+    """Kernels of different shared memory in turn (up to 1.9 times as long overlapped before)."""
+    import torch
+
+    steps = [_handle(sb, torch, rows, width, fmt, **kw) for rows, width, fmt, kw in order]
+    flag = torch.zeros(1, device="cuda")
+
+    def together():
+        for _, step in steps:
+            step()
+
+    def apart():
+        for _, step in steps:
+            step()
+            flag.fill_(1.0)
+
+    assert _per_step(torch, 100, together) <= _per_step(torch, 100, apart)
+
+
 @pytest.mark.parametrize("C,rows,width", [(64, 16554, 45), (64, 60000, 20), (128, 20000, 40), (32, 16554, 45)])
 def test_tiled_slices(sb, C, rows, width):
     """SELL-C-sigma on kernel 8: few long blocks a CTA (1.2 to 1.4 times as long overlapped before)."""
