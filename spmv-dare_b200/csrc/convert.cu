@@ -543,7 +543,7 @@ static const StagedTime * staged_time(const Handle & h)
 {
 	static const StagedTime naive{2.3, 70, 8.5, 1, 6.5, 0}, vec4{3.4, 80, 8.5, 1.2, 190, 1280}, vec8{4.4, 62, 12, 1.2, 230, 1280},
 			sell{2.4, 50, 6, 1, 6.5, 0}, sorted{3.4, 65, 6.5, 1.2, 6.5, 0}, f32{2, 60, 9.6, 1.7, 13, 0},
-			sellcs32{3.9, 1e9, 9, 1, 26, 0}, sellcs64{3.9, 1e9, 9, 1, 46, 0};
+			sellcs32{3.9, 1e9, 9, 1, 26, 0}, sellcs64{4.8, 1e9, 9, 1, 55, 0};
 	if (h.desc.values == SPMV_VALUES_F32)
 		return &f32;
 	switch (h.desc.format) {

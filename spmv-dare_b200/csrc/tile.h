@@ -45,7 +45,8 @@ struct LongUnit {
 
 // What the staged kernel that would run instead takes, beside a launch: its stored entries, each
 // `base` + (mean row length) / `per_length` ps, at most `most`, times `uneven` where the widest
-// slice is over twice the mean; or its longest row, from `chain_from` entries on, at `chain` ns an entry.
+// slice is over twice the mean; or its longest row, from `chain_from` entries on, at `chain` ns an entry
+// (both, where that is over eight times the mean).
 struct StagedTime {
 	double base, per_length, most, uneven, chain;
 	int chain_from;

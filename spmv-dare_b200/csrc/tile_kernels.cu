@@ -939,8 +939,9 @@ bool staged_takes_less(const StagedTime & k, bool f32, int64_t entries, int64_t 
 	double staged = entries * 1e-6 * std::min(k.base + mean / k.per_length, k.most);
 	if (widest > 2 * slice)
 		staged *= k.uneven;
-	if (longest > k.chain_from)
-		staged = std::max(staged, longest * k.chain * 1e-3);
+	const double chain = longest > k.chain_from ? longest * k.chain * 1e-3 : 0.0;
+	// far longer rows than the rest come together and wait for each other
+	staged = longest > 8 * mean ? staged + chain : std::max(staged, chain);
 	return staged < 0.95 * tiles;
 }
 
