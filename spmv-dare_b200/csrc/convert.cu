@@ -549,8 +549,11 @@ static const StagedTime * staged_time(const Handle & h)
 	switch (h.desc.format) {
 	case SPMV_FMT_CSR_NAIVE: return &naive;
 	case SPMV_FMT_CSR_VEC: return h.desc.vec_len == 8 ? &vec8 : &vec4;
-	case SPMV_FMT_SELL: return &sell;
-	case SPMV_FMT_SELL_SORTED: return &sorted;
+	case SPMV_FMT_SELL:
+	case SPMV_FMT_SELL_SORTED:
+		if (h.desc.vec_len >= 16)
+			return h.desc.vec_len <= 32 ? &sellcs32 : h.desc.vec_len <= 64 ? &sellcs64 : nullptr;
+		return h.desc.format == SPMV_FMT_SELL ? &sell : &sorted;
 	default: return h.desc.sellcs_c <= 32 ? &sellcs32 : h.desc.sellcs_c <= 64 ? &sellcs64 : nullptr;
 	}
 }
@@ -595,8 +598,8 @@ int build_exec(Handle & h, const int32_t * d_P, int64_t U, int V)
 		// block selects the staged kernels.
 		const bool sliced = h.desc.format == SPMV_FMT_SELL_C_S || h.desc.format == SPMV_FMT_SELL ||
 				h.desc.format == SPMV_FMT_SELL_SORTED;
-		if (h.tiles.slower && V <= 64)
-			k = 4;                  // what the row tiles were compared with
+		if (h.tiles.faster)
+			k = h.tiles.faster;     // what the row tiles were compared with
 		else if (sliced && V == 32 && h.desc.block_nnz == 0)
 			k = 10;
 		else

@@ -54,7 +54,7 @@ struct StagedTime {
 
 struct TilePlan {
 	bool built = false;
-	bool slower = false;         // not built: the staged kernel takes less time
+	int faster = 0;              // not built: the kernel that takes less time (4, 10)
 	int32_t pad_col = PAD_OWN;
 	bool f32 = false, mixed = false, wide = false, staged = false;
 	bool split = false;          // csr_naive arithmetic (MIXED batches: by slice)

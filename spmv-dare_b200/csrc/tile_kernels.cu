@@ -917,24 +917,31 @@ TileFn tile_fn(const TilePlan & p)
 	                : tile_kernel<Sum::FMA, DEEP_CTAS, true>;
 }
 
-// Whether the staged kernel takes less time.  Row tiles give a slice of 32 rows to a warp, which
+// The kernel that takes less time than row tiles, or 0.  Row tiles give a slice of 32 rows to a warp, which
 // waits for x tile by tile; below two slices a resident warp (190,000 rows on 148 SMs) the widest
 // slices are their time, and matrices of few long rows took up to eight times as long as on kernel 4
 // (2,000 rows of 2,000, SELL 35 us and 282; csr_naive 6,000 rows of 600 39 and 94, 40,000 of 100 18
 // and 26).  us an entry of the mean and of the widest slice by the slices an SM has: measured 0.14,
-// 0.18 and 0.23 with 1, 4 and 10 or more of even rows of 0.4 lines an entry, half of that with
+// 0.19 and 0.25 with 1, 4 and 12 or more of even rows of 0.4 lines an entry, half of that with
 // consecutive columns; 0.08 to 0.14 where a few are widest.
-bool staged_takes_less(const StagedTime & k, bool f32, int64_t entries, int64_t rows, int64_t stored, int64_t slices,
+//
+// Slices of 32 even rows of 100 entries and more have kernel 10 besides, whose warps take a slice at a
+// time at any size: 60,000 rows of 200 35 us (tiles 57, kernel 4 50), 120,000 of 100 37 (43, 49), 200,000
+// of 200 92 (103, 147); shorter or uneven rows are the tiles' (700,000 of 30 62 and 60).
+int faster_kernel(const StagedTime & k, int V, bool f32, int64_t entries, int64_t rows, int64_t stored, int64_t slices,
 		const int * stat, int num_sms)
 {
 	const int longest = stat[LONGEST], widest = stat[WIDEST];
-	if (slices >= (int64_t) num_sms * 2 * DEEP_CTAS * TILE_WARPS)
-		return false;
 	const double mean = (double) entries / rows, slice = (double) stored / (32 * slices), an_sm = (double) slices / num_sms;
+	const bool enough = slices >= (int64_t) num_sms * 2 * DEEP_CTAS * TILE_WARPS;
+	const bool ten = V == 32 && mean >= 96 && longest < 2 * mean;
+	if (enough && !ten)
+		return 0;
 	const double lines = std::min(1.0, 0.35 + 1.66 * stat[LINES] / std::max(stat[LINES_OF], 1));
-	const double even = lines * std::min(0.13 + 0.012 * an_sm, 0.23), few = lines * std::min(0.08 + 0.004 * an_sm, 0.13);
-	double tiles = stored * (f32 ? 1.6e-6 : 2.4e-6);
-	tiles = std::max(tiles, std::max(slice * even, widest * few));
+	const double even = lines * std::min(0.15 + 0.009 * an_sm, 0.25), few = lines * std::min(0.08 + 0.004 * an_sm, 0.13);
+	double tiles = stored * (f32 ? 1.6e-6 : 2.7e-6);
+	if (!enough)
+		tiles = std::max(tiles, std::max(slice * even, widest * few));
 	tiles = std::max(tiles, longest * 0.005);
 	double staged = entries * 1e-6 * std::min(k.base + mean / k.per_length, k.most);
 	if (widest > 2 * slice)
@@ -942,7 +949,12 @@ bool staged_takes_less(const StagedTime & k, bool f32, int64_t entries, int64_t 
 	const double chain = longest > k.chain_from ? longest * k.chain * 1e-3 : 0.0;
 	// far longer rows than the rest come together and wait for each other
 	staged = longest > 8 * mean ? staged + chain : std::max(staged, chain);
-	return staged < 0.95 * tiles;
+	if (ten) {
+		const double t = std::max(std::max(30.0, 7 + entries * 1.8e-6), widest * 0.09);
+		if (t < staged)
+			return t < 0.95 * tiles ? 10 : 0;
+	}
+	return staged < 0.95 * tiles && !enough ? 4 : 0;
 }
 
 int lay_out(TilePlan & p, const std::vector<TileSource> & src, int lanes, bool f32, bool mixed, const StagedTime * staged,
@@ -1023,8 +1035,9 @@ int lay_out(TilePlan & p, const std::vector<TileSource> & src, int lanes, bool f
 	const int nlong = stat[0];
 	if (total > INT32_MAX - 4096 || total > entries + entries / 3 + 65536)
 		return SPMV_OK;
-	p.slower = staged && staged_takes_less(*staged, f32, entries, rows, total, ns, stat, num_sms);
-	if (p.slower)
+	if (staged)
+		p.faster = faster_kernel(*staged, src[0].V, f32, entries, rows, total, ns, stat, num_sms);
+	if (p.faster)
 		return SPMV_OK;
 	const size_t vs = f32 ? sizeof(float) : sizeof(double);
 	SPMV_TRY(alloc((void **) &p.sptr, (ns + 1) * sizeof(int32_t)));
@@ -1106,9 +1119,9 @@ int build_tiles(TilePlan & p, const std::vector<TileSource> & src, int lanes, bo
 	if (!p.built) {
 		for (void * a : taken)
 			memory.drop(a);
-		const bool slower = p.slower;
+		const int faster = p.faster;
 		p = TilePlan();
-		p.slower = slower;
+		p.faster = faster;
 	}
 	if (st == SPMV_ERR_NOMEM) {
 		clear_error();

@@ -36,6 +36,18 @@ def test_few_long_rows(sb, orc, fmt, kw, m, k):
     assert _bits_equal(h.spmv(x, np.full(m, 1.0)), _expected(orc, fmt, kw, rp, ci, v, x))
 
 
+@pytest.mark.parametrize("fmt,kw", [("sell", dict(vec_len=32)), ("sell_sorted", dict(vec_len=32)), ("sell_c_s", {})])
+def test_long_even_rows_in_slices_of_32(sb, orc, fmt, kw):
+    m, k = 60003, 200
+    n = 28 * (k + 3)
+    rp, ci, v, x = _even(m, k, n, k)
+    h = sb.csr_to_format(rp, ci, v, m, n, int(rp[-1]), format=fmt, **kw)
+    assert h.exec_choice() == (10, 0)
+    if fmt == "sell_c_s":
+        kw = dict(sellcs_c=32, sellcs_sigma=512)
+    assert _bits_equal(h.spmv(x, np.full(m, 1.0)), _expected(orc, fmt, kw, rp, ci, v, x))
+
+
 @pytest.mark.parametrize("k", [21, 32, 47])
 @pytest.mark.parametrize("fmt,kw", FORMS)
 def test_rows_enough_for_the_chip(sb, orc, fmt, kw, k):
@@ -47,7 +59,7 @@ def test_rows_enough_for_the_chip(sb, orc, fmt, kw, k):
     assert _bits_equal(h.spmv(x, np.full(m, 1.0)), _expected(orc, fmt, kw, rp, ci, v, x))
 
 
-@pytest.mark.parametrize("m,k", SHAPES + [(16554, 45), (100001, 45)])
+@pytest.mark.parametrize("m,k", SHAPES + [(16554, 45), (100001, 45), (60003, 200), (200001, 200)])
 @pytest.mark.parametrize("fmt,kw,kernels", [("csr_naive", {}, (4,)), ("csr_naive", dict(value_type="f32"), (4,)),
                                             ("csr_vec", dict(vec_len=4), (4,)), ("sell", dict(vec_len=4), (4,)),
                                             ("sell_sorted", dict(vec_len=32), (10,)),

@@ -32,8 +32,8 @@ def test_a_matrix_without_room_for_the_layout(sb, fmt, kw, kernel):
     scratch of its reordering is as large, so the layout always finds its place.)"""
     import torch
 
-    csr = _device_matrix(torch, 20_000_000)
-    x = torch.rand(100000, dtype=torch.float64, device="cuda")
+    csr = _device_matrix(torch, 20_000_000, 400000)
+    x = torch.rand(400000, dtype=torch.float64, device="cuda")
     if "value_type" in kw:
         x = x.float()
     roomy = sb.csr_to_format(*csr, format=fmt, **kw)
