@@ -103,8 +103,9 @@ extern "C" {
  *                       (FP64 and FP32 CSR; not csr_vec with 1, 2 or 16 lanes, slices of 1 or 2 rows, nor a
  *                       matrix the layout would pad by more than a third); below 190,000 rows only
  *                       where kernel 4 would take longer by its rows' number and lengths, else that
- *                       (not with slices of more than 64 rows), and kernel 10 for slices of 32 long,
- *                       even rows where that takes less.
+ *                       (not with slices of more than 64 rows), kernel 10 for slices of 32 long, even
+ *                       rows where that takes less, and kernel 4 for csr_naive (FP64) rows of fewer
+ *                       than 12 entries on average.
  *                       Otherwise 10 for slices of 32 rows without a block_nnz, 8 for other
  *                       SELL-C-sigma, 4 for the others.  DIV-RF: the segment decoder up to 32
  *                       lanes (warps decode runs of a packet from places noted at

@@ -48,6 +48,10 @@ constexpr int TILE_WARPS = TILE_THREADS / 32;
 constexpr int TILE_WINDOW = 1024;       // rows sorted together
 constexpr int LONG_STEP = 256;          // entries a warp stages at a time of a long row
 constexpr int64_t SLICE_COST = 128;     // entries' worth of a slice's bookkeeping
+// csr_naive rows of fewer entries run kernel 4 at any size: it multiplies in its gather and adds from
+// consecutive shared memory, and tiles spend their time on slices (4 M rows of 6 86 us and 104, 2 M of 5
+// 38 and 45, 1 M of 9 28-36 and 31-40; 4 M of 13 136-182 and 130-177, 400,000 of 16 25 and 23).
+constexpr int64_t NAIVE_MEAN = 12;
 constexpr int64_t RANGE_COST = 2048;
 
 // ------------------------------------------------------------------ arithmetic of a row
@@ -977,6 +981,10 @@ int lay_out(TilePlan & p, const std::vector<TileSource> & src, int lanes, bool f
 		return SPMV_OK;
 	}
 	const int64_t mean = entries / rows;
+	if (staged && src[0].split && !f32 && mean < NAIVE_MEAN) {
+		p.faster = 4;
+		return SPMV_OK;
+	}
 	// From how many entries a row gets a warp of its own.  A lane adds 8 entries of its row in
 	// 0.3 us at best (2 us with every SM full), a warp of its own a row in 3 us and 5 ns an entry.
 	// Launches of 10 us and more (12 bytes an entry at 6 TB/s): rows that would take a lane about

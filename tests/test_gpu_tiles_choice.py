@@ -48,6 +48,17 @@ def test_long_even_rows_in_slices_of_32(sb, orc, fmt, kw):
     assert _bits_equal(h.spmv(x, np.full(m, 1.0)), _expected(orc, fmt, kw, rp, ci, v, x))
 
 
+@pytest.mark.parametrize("m,k", [(2000001, 5), (600000, 9)])
+def test_short_rows_of_csr_naive(sb, orc, m, k):
+    """Kernel 4 at any size (row tiles took 1.1 to 1.2 times as long)."""
+    rp, ci, v, x = _even(m, k, 28 * (k + 3), k)
+    args = (rp, ci, v, m, x.size, int(rp[-1]))
+    h, named = sb.csr_to_format(*args, format="csr_naive"), sb.csr_to_format(*args, format="csr_naive", kernel=4)
+    assert h.exec_choice() == (4, 0)
+    assert h.device_bytes == named.device_bytes
+    assert _bits_equal(h.spmv(x, np.full(m, 1.0)), orc.csr_spmv(rp, ci, v, x))
+
+
 @pytest.mark.parametrize("k", [21, 32, 47])
 @pytest.mark.parametrize("fmt,kw", FORMS)
 def test_rows_enough_for_the_chip(sb, orc, fmt, kw, k):
