@@ -747,22 +747,21 @@ __global__ void __launch_bounds__(TILE_WINDOW / 2) tile_sort_kernel(TileSource s
 	}
 }
 
-// Rows of at least (i + 2) / 2 x mean entries (and 32), i = 0 .. 5, among the source's.
+// Rows of at least so many entries, among the source's.
 constexpr int CENSUS = 6;
-__host__ __device__ __forceinline__ int64_t census_length(int i, int64_t mean)
-{
-	const int64_t t = (i + 2) * mean / 2;
-	return t > 32 ? t : 32;
-}
-__global__ void long_census_kernel(TileSource s, int64_t mean, int * count)
+struct Census {
+	int64_t length[CENSUS];
+};
+__global__ void long_census_kernel(TileSource s, Census c, int * count)
 {
 	const int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
 	int64_t start;
 	int stride, cnt = 0;
 	if (i < s.m)
 		source_row(s, i, start, stride, cnt);
+	#pragma unroll
 	for (int k = 0; k < CENSUS; k++) {
-		const unsigned b = __ballot_sync(0xffffffffu, i < s.m && cnt >= census_length(k, mean));
+		const unsigned b = __ballot_sync(0xffffffffu, i < s.m && cnt >= c.length[k]);
 		if ((threadIdx.x & 31) == 0 && b)
 			atomicAdd(count + k, __popc(b));
 	}
@@ -993,23 +992,31 @@ int lay_out(TilePlan & p, const std::vector<TileSource> & src, int lanes, bool f
 	// longest rows alone: as many long rows as the chip holds warps beside the slices.
 	DevBuf cnt;
 	SPMV_TRY(cnt.alloc((STATS + CENSUS) * sizeof(int), s));
-	SPMV_CUDA_TRY(cudaMemsetAsync(cnt.p, 0, (STATS + CENSUS) * sizeof(int), s));
 	const int64_t us = 4 + entries * 12 / 6000000;
 	int64_t lm = 2 * us < 512 ? 2 * us : 512;
 	lm = lm > 4 * mean ? lm : 4 * mean;
 	lm = lm > 32 ? lm : 32;
-	if (us < 10) {
-		int census[CENSUS];
+	const bool brief = us < 10;
+	auto count_rows = [&](const Census & c, int (&rows_of)[CENSUS]) -> int {
+		SPMV_CUDA_TRY(cudaMemsetAsync(cnt.as<int>() + STATS, 0, sizeof(rows_of), s));
 		for (const TileSource & t : src) {
 			if (t.m > 0)
-				long_census_kernel<<<(unsigned) ceil_div(t.m, 256), 256, 0, s>>>(t, mean, cnt.as<int>() + STATS);
+				long_census_kernel<<<(unsigned) ceil_div(t.m, 256), 256, 0, s>>>(t, c, cnt.as<int>() + STATS);
 			SPMV_CUDA_TRY(cudaGetLastError());
 		}
-		SPMV_CUDA_TRY(cudaMemcpyAsync(census, cnt.as<int>() + STATS, sizeof(census), cudaMemcpyDeviceToHost, s));
+		SPMV_CUDA_TRY(cudaMemcpyAsync(rows_of, cnt.as<int>() + STATS, sizeof(rows_of), cudaMemcpyDeviceToHost, s));
 		SPMV_CUDA_TRY(cudaStreamSynchronize(s));
+		return SPMV_OK;
+	};
+	Census c;
+	int census[CENSUS];
+	if (brief) {
+		for (int i = 0; i < CENSUS; i++)
+			c.length[i] = std::max((i + 2) * mean / 2, (int64_t) 32);
+		SPMV_TRY(count_rows(c, census));
 		for (int i = 0; i < CENSUS; i++)
 			if (census[i] + ns <= (int64_t) num_sms * DEEP_CTAS * TILE_WARPS) {
-				lm = census_length(i, mean);
+				lm = c.length[i];
 				break;
 			}
 	}
@@ -1027,19 +1034,39 @@ int lay_out(TilePlan & p, const std::vector<TileSource> & src, int lanes, bool f
 	SPMV_TRY(sptr64.alloc((ns + 1) * sizeof(int64_t), s));
 	SPMV_TRY(alloc((void **) &p.slot_row, nslots * sizeof(int32_t)));
 	SPMV_TRY(alloc((void **) &p.slot_cnt, nslots * sizeof(int32_t)));
-	for (size_t i = 0; i < src.size(); i++) {
-		if (src[i].m == 0)
-			continue;
-		tile_sort_kernel<<<(unsigned) ceil_div(src[i].m, TILE_WINDOW), TILE_WINDOW / 2, 0, s>>>(src[i], long_min[i], slot0[i],
-				ceil_div(src[i].m, 32) * 32, d_src.as<int32_t>(), p.slot_row, p.slot_cnt, width.as<int64_t>(), cnt.as<int>());
-		SPMV_CUDA_TRY(cudaGetLastError());
-	}
-	SPMV_TRY(scan_exclusive(width.as<int64_t>(), sptr64.as<int64_t>(), ns, s));
 	int64_t total = 0;
 	int stat[STATS];
-	SPMV_CUDA_TRY(cudaMemcpyAsync(&total, sptr64.as<int64_t>() + ns, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-	SPMV_CUDA_TRY(cudaMemcpyAsync(stat, cnt.p, sizeof(stat), cudaMemcpyDeviceToHost, s));
-	SPMV_CUDA_TRY(cudaStreamSynchronize(s));
+	for (int pass = 0;; pass++) {
+		SPMV_CUDA_TRY(cudaMemsetAsync(cnt.p, 0, STATS * sizeof(int), s));
+		for (size_t i = 0; i < src.size(); i++) {
+			if (src[i].m == 0)
+				continue;
+			tile_sort_kernel<<<(unsigned) ceil_div(src[i].m, TILE_WINDOW), TILE_WINDOW / 2, 0, s>>>(src[i], long_min[i], slot0[i],
+					ceil_div(src[i].m, 32) * 32, d_src.as<int32_t>(), p.slot_row, p.slot_cnt, width.as<int64_t>(), cnt.as<int>());
+			SPMV_CUDA_TRY(cudaGetLastError());
+		}
+		SPMV_TRY(scan_exclusive(width.as<int64_t>(), sptr64.as<int64_t>(), ns, s));
+		SPMV_CUDA_TRY(cudaMemcpyAsync(&total, sptr64.as<int64_t>() + ns, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+		SPMV_CUDA_TRY(cudaMemcpyAsync(stat, cnt.p, sizeof(stat), cudaMemcpyDeviceToHost, s));
+		SPMV_CUDA_TRY(cudaStreamSynchronize(s));
+		// Many long rows in a longer launch of one matrix: once more with the length from which the warps
+		// of the long ones (3.2 us each) and the wait for the widest slice take least (csr_vec, 1 M rows of 12,
+		// exponential lengths: 9,400 rows from 56 entries on 67 us, 900 from 84 on 54).
+		const double warps_us = 3.2 / (num_sms * DEEP_CTAS), entry_us = 0.13;
+		if (pass > 0 || brief || src.size() > 1 || stat[0] * warps_us < lm / 2 * entry_us)
+			break;
+		for (int i = 0; i < CENSUS; i++)
+			c.length[i] = (i + 3) * lm / 2;
+		SPMV_TRY(count_rows(c, census));
+		double least = stat[0] * warps_us + lm * entry_us;
+		for (int i = 0; i < CENSUS; i++)
+			if (census[i] * warps_us + c.length[i] * entry_us < least) {
+				least = census[i] * warps_us + c.length[i] * entry_us;
+				long_min[0] = (int) std::min(c.length[i], (int64_t) ((1 << 21) - 3));
+			}
+		if (long_min[0] == lm)
+			break;
+	}
 	const int nlong = stat[0];
 	if (total > INT32_MAX - 4096 || total > entries + entries / 3 + 65536)
 		return SPMV_OK;

@@ -48,6 +48,22 @@ def test_long_even_rows_in_slices_of_32(sb, orc, fmt, kw):
     assert _bits_equal(h.spmv(x, np.full(m, 1.0)), _expected(orc, fmt, kw, rp, ci, v, x))
 
 
+@pytest.mark.parametrize("fmt,kw", [f for f in FORMS if f[0] != "csr_naive"])
+def test_many_longer_rows(sb, orc, fmt, kw):
+    """Exponential lengths: thousands of rows above the first bound of rows with a warp of their own."""
+    r = np.random.default_rng(11)
+    m, n = 700003, 30000
+    lengths = r.exponential(14.0, m).astype(np.int64)
+    rp = np.zeros(m + 1, np.int32)
+    np.cumsum(lengths, out=rp[1:])
+    start = (r.random(m) * (n - 20 * lengths)).astype(np.int64)
+    ci = (np.repeat(start, lengths) + 20 * (np.arange(rp[-1]) - np.repeat(rp[:-1], lengths))).astype(np.int32)
+    v, x = r.uniform(-1, 1, rp[-1]), r.uniform(-1, 1, n)
+    h = sb.csr_to_format(rp, ci, v, m, n, int(rp[-1]), format=fmt, **kw)
+    assert h.exec_choice()[0] == 11
+    assert _bits_equal(h.spmv(x, np.full(m, 1.0)), _expected(orc, fmt, kw, rp, ci, v, x))
+
+
 @pytest.mark.parametrize("m,k", [(2000001, 5), (600000, 9)])
 def test_short_rows_of_csr_naive(sb, orc, m, k):
     """Kernel 4 at any size (row tiles took 1.1 to 1.2 times as long)."""
